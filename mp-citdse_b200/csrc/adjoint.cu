@@ -32,9 +32,8 @@
 // stage inputs y_s and norms, then walks it backwards.  Cost: one forward,
 // one recomputed forward, one adjoint sweep (about 3 forwards).  When the
 // couplings fit in shared memory (the resident path) each pass is one
-// persistent launch (resident.cu: the forward with checkpoint / segment
-// outputs, and k_adj_resident for the sweep); otherwise the streamed kernels
-// below run step by step.
+// persistent launch (resident.cu, on the Horner form of the step); otherwise
+// the streamed kernels below run step by step.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -283,11 +282,11 @@ struct mpc_adjoint_state {
   double2* segX = nullptr;    // [ckpt + 1][ntot]
   double2* segY = nullptr;    // [ckpt][13][ntot]  (slot 0 unused: y_0 = x_n)
   double* segN = nullptr;     // [ckpt]
-  // a second segment buffer set for the fused reverse pass (recompute of one
-  // segment while the previous one is swept), allocated on first use
-  double2* segX2 = nullptr;
+  // resident passes: a second segment buffer set (recompute of one segment
+  // while the one after it is swept) and every step's norm, allocated on
+  // first use; a segment's slots hold its Horner vectors and states
   double2* segY2 = nullptr;
-  double* segN2 = nullptr;
+  double* norms = nullptr;
   double2* lam = nullptr;
   double2* zbar = nullptr;
   double2* v = nullptr;
@@ -353,6 +352,13 @@ int ensure_adjoint(mpc_ctx* c, int steps, int ckpt) {
   a->cap_seg = ckpt;
   a->cap_steps = steps;
   return MPC_OK;
+}
+
+int ensure_resident(mpc_adjoint_state* a, size_t n) {
+  int rc = MPC_OK;
+  if (!a->segY2) rc = aalloc(a, &a->segY2, n * a->cap_seg * kNumStages);
+  if (!rc && !a->norms) rc = aalloc(a, &a->norms, a->cap_steps);
+  return rc;
 }
 
 // One forward step from x (stage inputs into ys[1..12], x_new into ys[13]),
@@ -427,10 +433,13 @@ int mpc_objective(mpc_ctx* c, const mpc_pulse* p, int K, const double* u, double
   const double2* x = a->ckpts;
   a->resident = mpc_use_resident(c) && mpc_resident_adjoint_ok(c);
   if (a->resident) {
-    // one persistent launch; it stores the checkpoints as it passes them
-    if ((rc = mpc_resident_forward_ex(c, a->ckpts, a->ckpts + n * a->nseg, c->d_Ftab, dt, steps,
-                                      nullptr, nullptr, nullptr, a->ckpts, ckpt_every,
-                                      (long long)n)))
+    // one persistent launch; it stores the checkpoints as it passes them, and
+    // the last segment's vectors, which the reverse pass then need not recompute
+    if ((rc = ensure_resident(a, n)) ||
+        (rc = mpc_resident_forward_ex(c, a->ckpts, a->ckpts + n * a->nseg, c->d_Ftab, dt, steps,
+                                      a->norms, a->ckpts, ckpt_every,
+                                      ((a->nseg - 1) & 1) ? a->segY2 : a->segY,
+                                      (a->nseg - 1) * ckpt_every, (long long)n)))
       return rc;
   } else {
     // the last segment keeps every state, stage input and norm as the reverse
@@ -457,7 +466,7 @@ int mpc_objective(mpc_ctx* c, const mpc_pulse* p, int K, const double* u, double
     CK(cudaMemcpyAsync(a->ckpts + n * a->nseg, a->segX + n * (steps - n0_last),
                        sizeof(double2) * n, cudaMemcpyDeviceToDevice, c->stream));
   }
-  a->last_kept = !a->resident;
+  a->last_kept = true;
   // objective on the host from x_N
   std::vector<double> xN(2 * c->g.ntot), eps(c->g.ntot);
   CK(cudaMemcpyAsync(xN.data(), a->ckpts + n * a->nseg, nb, cudaMemcpyDeviceToHost, c->stream));
@@ -502,9 +511,13 @@ int mpc_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
   const int ntot = c->g.ntot;
   const int nbk = (ntot + 255) / 256;
   int rc;
-  k_adj_seed<<<nbk, 256, 0, c->stream>>>(a->ckpts + n * nseg, c->d_eps, a->lam, a->target,
-                                    c->yield_thr, ntot);
-  CK(cudaGetLastError());
+  if (a->resident) {
+    if ((rc = mpc_resident_seed(c, a->ckpts + n * nseg, a->lam, a->target))) return rc;
+  } else {
+    k_adj_seed<<<nbk, 256, 0, c->stream>>>(a->ckpts + n * nseg, c->d_eps, a->lam, a->target,
+                                           c->yield_thr, ntot);
+    CK(cudaGetLastError());
+  }
   AdjCombineArgs ac{};
   ac.v = a->v;
   ac.zbar = a->zbar;
@@ -519,35 +532,17 @@ int mpc_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
   ac.gauge = (c->gauge == 'l') ? 0 : 1;
   ac.h = dt;
   ac.g = c->g;
-  if (a->resident && mpc_resident_fused_ok(c)) {
+  if (a->resident) {
     // one persistent launch: each segment's recompute runs concurrently with
     // the sweep of the segment after it
-    if (!a->segX2) {
-      if ((rc = aalloc(a, &a->segX2, n * (ckpt + 1))) ||
-          (rc = aalloc(a, &a->segY2, n * (size_t)ckpt * kNumStages)) ||
-          (rc = aalloc(a, &a->segN2, ckpt)))
-        return rc;
-    }
-    double2* sx[2] = {a->segX, a->segX2};
-    double2* sy[2] = {a->segY, a->segY2};
-    double* sn[2] = {a->segN, a->segN2};
-    if ((rc = mpc_resident_backward_fused(c, a->ckpts, steps, ckpt, c->d_Ftab, dt, sx, sy, sn,
-                                          a->lam, a->fbar, (long long)n)))
+    double2* sv[2] = {a->segY, a->segY2};
+    if ((rc = mpc_resident_backward(c, a->ckpts, a->norms, steps, ckpt, c->d_Ftab, dt, sv,
+                                    a->last_kept, a->lam, a->fbar, (long long)n)))
       return rc;
   }
-  for (int seg = nseg - 1; seg >= 0 && !(a->resident && mpc_resident_fused_ok(c)); --seg) {
+  for (int seg = nseg - 1; seg >= 0 && !a->resident; --seg) {
     const int n0 = seg * ckpt;
     const int len = std::min(ckpt, steps - n0);
-    if (a->resident) {
-      // recompute the segment (states, stage inputs, norms), then its sweep
-      if ((rc = mpc_resident_forward_ex(c, a->ckpts + n * seg, a->segX + n * len,
-                                        c->d_Ftab + n0, dt, len, a->segX, a->segY, a->segN,
-                                        nullptr, 0, (long long)n)) ||
-          (rc = mpc_resident_adjoint(c, c->d_Ftab + n0, dt, len, a->segX, a->segY, a->segN,
-                                     a->lam, a->fbar + n0, (long long)n)))
-        return rc;
-      continue;
-    }
     // recompute the segment, keeping states, stage inputs and norms (the
     // forward kept the last one)
     const bool kept = a->last_kept && seg == nseg - 1;

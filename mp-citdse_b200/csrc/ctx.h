@@ -162,18 +162,12 @@ int mpc_resident_run(mpc_ctx* c, double dt, int steps, int pop_index);
 bool mpc_use_resident(mpc_ctx* c);  // the resident path applies (set-up done, not disabled)
 bool mpc_resident_adjoint_ok(mpc_ctx* c);
 int mpc_resident_forward_ex(mpc_ctx* c, const double2* x_in, double2* x_out, const double* Ftab,
-                            double dt, int steps, double2* seg_x, double2* seg_y,
-                            double* norm_hist, double2* ckpt, int ckpt_every, long long vpitch);
-int mpc_resident_adjoint(mpc_ctx* c, const double* Ftab, double dt, int len,
-                         const double2* seg_x, const double2* seg_y, const double* seg_n,
-                         double2* lam, double* fbar, long long vpitch);
-// The fused reverse pass (recompute of one segment concurrent with the sweep
-// of the next, one persistent launch; resident.cu).
-bool mpc_resident_fused_ok(mpc_ctx* c);
-int mpc_resident_backward_fused(mpc_ctx* c, const double2* ckpts, int steps, int ckpt_every,
-                                const double* Ftab, double dt, double2* const* segX,
-                                double2* const* segY, double* const* segN, double2* lam,
-                                double* fbar, long long vpitch);
+                            double dt, int steps, double* norm_hist, double2* ckpt,
+                            int ckpt_every, double2* seg_v, int seg_from, long long vpitch);
+int mpc_resident_backward(mpc_ctx* c, const double2* ckpt, const double* norms, int steps,
+                          int ckpt_every, const double* Ftab, double dt, double2* const* seg_v,
+                          bool last_kept, double2* lam, double* fbar, long long vpitch);
+int mpc_resident_seed(mpc_ctx* c, const double2* x, double2* lam, int target);
 
 // Launch helpers of the single-pulse path (mpc_tdse.cu), used by adjoint.cu.
 int mpc_launch_stream(mpc_ctx* c, const double2* y);
