@@ -32,6 +32,7 @@
 #include "batch_tma.cuh"
 #include "batch_types.h"
 #include "ctx.h"
+#include "flow_batch.h"
 #include "dev_util.cuh"
 #include "plan.h"
 #include "rkf78.h"
@@ -1170,6 +1171,9 @@ int mpc_batch_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
                     "dt*max|E| = %.4g exceeds the RKF78 imaginary-axis stability bound %.4g",
                     dt * c->eps_max, kRk78ImagStability);
   CK(cudaSetDevice(c->device));
+  if (mpc_flowb_wanted(c, B))
+    return mpc_flowb_advance(c, B, pulses, t0, dt, steps, pop_index, ct, pop_out, norm_out,
+                             max_steps);
   FixedStep fx{};
   fx.on = 1;
   fx.dt = dt;

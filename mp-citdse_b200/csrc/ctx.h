@@ -82,6 +82,7 @@ struct mpc_ctx {
   struct mpc_resident_state* resident = nullptr;  // resident path (resident.cu)
   struct mpc_batch_res_state* batch_res = nullptr;  // resident batched path (batch_resident.cu)
   struct mpc_badj_state* badj = nullptr;  // batched objective / adjoint (batch_adjoint.cu)
+  struct mpc_flowb_state* flowb = nullptr;  // persistent batched path (flow_batch.cu)
   int path = 0;  // 0 automatic, 1 streaming, 2 resident (MPC_PATH_*)
   double yield_thr = 0.0;  // yield objective: 1 - sum over states below this energy
   // MPC_BATCH_VARIANT=v at context creation pins the stage-GEMM tile variant
@@ -150,6 +151,7 @@ struct ProfScope {
 
 void mpc_batch_free(mpc_ctx* c);
 void mpc_adjoint_free(mpc_ctx* c);
+bool mpc_allow_smem(const void* fn, int optin);
 bool mpc_resident_setup(mpc_ctx* c);
 void mpc_resident_free(mpc_ctx* c);
 void mpc_batch_res_free(mpc_ctx* c);

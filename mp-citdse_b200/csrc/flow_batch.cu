@@ -1,0 +1,343 @@
+// flow_batch.cu -- host side of the persistent batched kernels
+// (flow_batch.cuh): the split of the rows over the CTAs and of the pulses
+// over column groups and chunks, the work space, the launches.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdlib>
+#include <numeric>
+#include <vector>
+
+#include "batch_types.h"
+#include "ctx.h"
+#include "flow_batch.cuh"
+#include "flow_batch.h"
+
+using namespace mpc;
+
+namespace {
+
+constexpr int kMaxGroups = 4;
+
+int window_len(const Geometry& g, int L) {
+  return (L > 0 ? g.state_off[L] - g.state_off[L - 1] : 0) +
+         (L < g.nblk ? g.state_off[L + 2] - g.state_off[L + 1] : 0);
+}
+
+// The kernels' instances, 8-row tiles x groups of 4 window rows per warp (the
+// cases of k_flow_batch's switch); a CTA takes the cheapest that holds its rows.
+struct FbConfig {
+  int mt, kt;
+};
+const FbConfig kConfigs[] = {{1, 6},  {2, 6},  {4, 6},  {2, 10}, {4, 10}, {6, 10},
+                             {2, 13}, {5, 13}, {2, 19}, {3, 19}, {2, 25}, {3, 25}};
+
+int config_for(int rows, int K) {
+  int best = -1;
+  for (int i = 0; i < (int)(sizeof kConfigs / sizeof kConfigs[0]); ++i) {
+    const FbConfig& f = kConfigs[i];
+    if (rows > 8 * f.mt || K > 4 * FW * f.kt) continue;
+    if (best < 0 || f.mt * f.kt < kConfigs[best].mt * kConfigs[best].kt) best = i;
+  }
+  return best;
+}
+// its DMMA work: the window groups that are there, all tiles of the instance
+int config_cost(int i, int K) { return kConfigs[i].mt * ((K + 4 * FW - 1) / (4 * FW)); }
+
+// One column group's CTAs: every block starts with the fewest CTAs whose
+// registers hold its rows; then the block whose CTAs cost most gets as many
+// more as its next cheaper instance needs, while there are any.
+bool split_group(const Geometry& g, int gp, std::vector<FbCta>& ctas, int* cost) {
+  const int nb = g.nstate_blk;
+  std::vector<int> cnt(nb), cfg(nb);
+  int used = 0;
+  for (int L = 0; L < nb; ++L) {
+    const int nL = g.state_off[L + 1] - g.state_off[L], K = window_len(g, L);
+    cnt[L] = 0;
+    for (int n = 1; n <= std::min(nL, gp) && !cnt[L]; ++n) {
+      cfg[L] = config_for((nL + n - 1) / n, K);
+      if (cfg[L] >= 0) cnt[L] = n;
+    }
+    if (!cnt[L]) return false;
+    used += cnt[L];
+  }
+  if (used > gp) return false;
+  auto work = [&](int L) { return config_cost(cfg[L], window_len(g, L)); };
+  while (true) {
+    int top = 0;
+    for (int L = 1; L < nb; ++L)
+      if (work(L) > work(top)) top = L;
+    const int nL = g.state_off[top + 1] - g.state_off[top], K = window_len(g, top);
+    int n = cnt[top] + 1, f = -1;
+    for (; n <= nL && used - cnt[top] + n <= gp; ++n) {
+      f = config_for((nL + n - 1) / n, K);
+      if (f >= 0 && config_cost(f, K) < work(top)) break;
+      f = -1;
+    }
+    if (f < 0) break;
+    used += n - cnt[top];
+    cnt[top] = n;
+    cfg[top] = f;
+  }
+  ctas.clear();
+  *cost = 0;
+  for (int L = 0; L < nb; ++L) {
+    const int o = g.state_off[L], nL = g.state_off[L + 1] - o;
+    for (int j = 0; j < cnt[L]; ++j) {
+      const int r0 = (int)((long long)nL * j / cnt[L]), r1 = (int)((long long)nL * (j + 1) / cnt[L]);
+      ctas.push_back({L, o + r0, r1 - r0, 0, (int)ctas.size(), cfg[L]});
+    }
+    *cost = std::max(*cost, work(L));
+  }
+  return true;
+}
+
+// Microseconds of a product for the chunks of one column group: items of 64
+// cycles per unit of DMMA work and about 2,500 for loads, sums and the rest
+// (1752 states 5,750 cycles at 57 units, 3492 states 8,000 at 75, 500 states
+// 3,100 at 14), or the exchange, about 4,500, when there are too few chunks to
+// hide it.
+double product_us(int cost, int chunks_per_group) {
+  return std::max(chunks_per_group * (64.0 * cost + 2500.0), 64.0 * cost + 4500.0) / 1900.0;
+}
+
+// The stage GEMM's product at B pulses: measured 47 us at 1752 states and 256
+// pulses, 23 at 64; 103 and 44 at 3492 states; 17 at 500 states and 256 pulses.
+double gemm_us(const Geometry& g, int B) {
+  double s = 0.0;
+  for (int L = 0; L < g.nblk; ++L) s += (double)g.blk[L].nrow * g.blk[L].ncol;
+  return 14.0 + 8.0 * s * B / 26e6;
+}
+
+struct Group {
+  bool ok = false;
+  int gp = 0;       // CTAs per group
+  int cost = 0;
+  FbCta* ctas = nullptr;
+};
+
+template <class T>
+int grow(T** p, size_t* cap, size_t n) {
+  if (*cap >= n) return MPC_OK;
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+  CK(cudaMalloc(p, sizeof(T) * n));
+  *cap = n;
+  return MPC_OK;
+}
+
+}  // namespace
+
+struct mpc_flowb_state {
+  bool tried = false, ok = false;
+  Group grp[kMaxGroups + 1];
+  // work space, kept between calls and grown on demand
+  double2* V = nullptr;
+  size_t V_n = 0;
+  double* part = nullptr;
+  size_t part_n = 0;
+  unsigned long long* ctr = nullptr;
+  size_t ctr_n = 0;
+  double2* xst = nullptr;
+  size_t xst_n = 0;
+  double2* io = nullptr;     // start and final states by pulse id
+  size_t io_n = 0;
+  int* ints = nullptr;       // chunk ids, chunk steps, pulse steps
+  size_t ints_n = 0;
+  mpc_pulse* pulse = nullptr;
+  size_t pulse_n = 0;
+  double* t0 = nullptr;
+  size_t t0_n = 0;
+  double* hist = nullptr;    // population and norm histories
+  size_t hist_n = 0;
+};
+
+bool mpc_flowb_setup(mpc_ctx* c) {
+  if (!c->flowb) c->flowb = new mpc_flowb_state();
+  mpc_flowb_state* f = c->flowb;
+  if (f->tried) return f->ok;
+  f->tried = true;
+  if (std::getenv("MPC_NO_RESIDENT")) return false;
+  int coop = 0, optin = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  if (!coop) return false;
+  if (cudaMemcpyToSymbol(f_G, rkf78::G, sizeof rkf78::G) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (int ng = 1; ng <= kMaxGroups; ++ng) {
+    Group& g = f->grp[ng];
+    std::vector<FbCta> one, all;
+    if (!split_group(c->g, c->num_sms / ng, one, &g.cost)) continue;
+    g.gp = (int)one.size();
+    for (int k = 0; k < ng; ++k)
+      for (FbCta t : one) {
+        t.grp = k;
+        all.push_back(t);
+      }
+    int per_sm = 0;
+    if (!mpc_allow_smem((const void*)&k_flow_batch<0>, optin) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flow_batch<0>, FTHREADS,
+                                                      flowb_smem()) != cudaSuccess ||
+        per_sm < 1 || cudaMalloc(&g.ctas, sizeof(FbCta) * all.size()) != cudaSuccess ||
+        cudaMemcpy(g.ctas, all.data(), sizeof(FbCta) * all.size(), cudaMemcpyHostToDevice) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    g.ok = true;
+    f->ok = true;
+  }
+  return f->ok;
+}
+
+void mpc_flowb_free(mpc_ctx* c) {
+  if (!c || !c->flowb) return;
+  mpc_flowb_state* f = c->flowb;
+  for (Group& g : f->grp) cudaFree(g.ctas);
+  cudaFree(f->V);
+  cudaFree(f->part);
+  cudaFree(f->ctr);
+  cudaFree(f->xst);
+  cudaFree(f->io);
+  cudaFree(f->ints);
+  cudaFree(f->pulse);
+  cudaFree(f->t0);
+  cudaFree(f->hist);
+  delete f;
+  c->flowb = nullptr;
+}
+
+namespace {
+
+// The column groups for nch chunks.
+int pick_groups(const mpc_flowb_state* f, int nch) {
+  int best = 0;
+  double t = 1e300;
+  for (int ng = 1; ng <= kMaxGroups; ++ng) {
+    if (!f->grp[ng].ok || ng > nch) continue;
+    const double x = product_us(f->grp[ng].cost, (nch + ng - 1) / ng);
+    if (x < t) {
+      t = x;
+      best = ng;
+    }
+  }
+  return best ? best : 1;
+}
+
+}  // namespace
+
+// Whether B pulses run faster here than on the stage GEMM.
+bool mpc_flowb_wanted(mpc_ctx* c, int B) {
+  if (c->path == MPC_PATH_STREAMING || !mpc_flowb_setup(c)) return false;
+  const mpc_flowb_state* f = c->flowb;
+  const int nch = (B + CP - 1) / CP, ng = pick_groups(f, nch);
+  return f->grp[ng].ok && product_us(f->grp[ng].cost, (nch + ng - 1) / ng) <= gemm_us(c->g, B);
+}
+
+// The fixed-step propagation of B pulses (mpc_batch_advance): ct host [B][n]
+// in and out; pop_out / norm_out host, rows of `ld` and ld - 1 (or null).
+int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
+                      const int* steps, int pop_index, double* ct, double* pop_out,
+                      double* norm_out, int max_steps) {
+  mpc_flowb_state* f = c->flowb;
+  const int n = c->g.ntot;
+  int rc;
+  // pulses by length, so that a chunk's end together
+  std::vector<int> order(B);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return steps[x] > steps[y]; });
+  const int nch_all = (B + CP - 1) / CP;
+  const long long ld = (long long)max_steps + 1;
+  const size_t hist = (size_t)B * ld;
+  std::vector<int> ints((size_t)nch_all * (CP + 1) + B, -1);
+  int* cid = ints.data();
+  int* cst = cid + (size_t)nch_all * CP;
+  int* ns = cst + nch_all;
+  for (int i = 0; i < B; ++i) cid[i] = order[i];
+  for (int k = 0; k < nch_all; ++k) cst[k] = steps[order[(size_t)k * CP]];
+  std::copy(steps, steps + B, ns);
+  if ((rc = grow(&f->ints, &f->ints_n, ints.size())) || (rc = grow(&f->pulse, &f->pulse_n, (size_t)B)) ||
+      (rc = grow(&f->t0, &f->t0_n, (size_t)B)) || (rc = grow(&f->io, &f->io_n, 2 * (size_t)B * n)) ||
+      (rc = grow(&f->hist, &f->hist_n, (pop_out ? hist : 0) + (norm_out ? hist : 0) + 1)))
+    return rc;
+  double2* in = f->io;
+  double2* out = f->io + (size_t)B * n;
+  CK(cudaMemcpyAsync(in, ct, sizeof(double2) * (size_t)B * n, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->ints, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(f->pulse, pulses, sizeof(mpc_pulse) * B, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->t0, t0, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
+  FbArgs a{};
+  a.D = c->d_D;
+  a.eps = c->d_eps;
+  a.slots = kFixSlots;
+  a.status = c->d_status;
+  a.in = in;
+  a.out = out;
+  a.pulse = f->pulse;
+  a.t0 = f->t0;
+  a.nsteps = f->ints + (ns - cid);
+  a.dt = dt;
+  a.gauge = (c->gauge == 'l') ? 0 : 1;
+  a.pop_index = pop_index;
+  a.hist_ld = ld;
+  a.pop_hist = pop_out ? f->hist : nullptr;
+  a.norm_hist = norm_out ? f->hist + (pop_out ? hist : 0) : nullptr;
+  a.g = c->g;
+  // launches of at most kMaxChunks chunks per column group
+  for (int k0 = 0; k0 < nch_all;) {
+    const int ng = pick_groups(f, nch_all - k0);
+    const Group& grp = f->grp[ng];
+    const int nch = std::min(nch_all - k0, kMaxChunks * ng);
+    const size_t vn = (size_t)nch * kFixSlots * n * CP, pn = (size_t)nch * 2 * grp.gp * 2 * CP;
+    if ((rc = grow(&f->V, &f->V_n, vn)) || (rc = grow(&f->part, &f->part_n, pn)) ||
+        (rc = grow(&f->ctr, &f->ctr_n, (size_t)nch)) ||
+        (rc = grow(&f->xst, &f->xst_n, (size_t)nch * n * CP)))
+      return rc;
+    CK(cudaMemsetAsync(f->V, 0xff, sizeof(double2) * vn, c->stream));
+    CK(cudaMemsetAsync(f->part, 0xff, sizeof(double) * pn, c->stream));
+    CK(cudaMemsetAsync(f->ctr, 0, sizeof(unsigned long long) * nch, c->stream));
+    a.cta = grp.ctas;
+    a.gp = grp.gp;
+    a.ng = ng;
+    a.nch = nch;
+    a.cid = f->ints + (size_t)k0 * CP;
+    a.csteps = f->ints + (cst - cid) + k0;
+    a.V = f->V;
+    a.part = f->part;
+    a.ctr = f->ctr;
+    a.xst = f->xst;
+    a.bc = mpc_barrier_cfg(c);
+    void* args[] = {&a};
+    ProfScope ps(c, MPC_KERNEL_BATCH_STAGE);
+    CK(cudaLaunchCooperativeKernel((const void*)&k_flow_batch<0>, dim3(ng * grp.gp),
+                                   dim3(FTHREADS), args, flowb_smem(), c->stream));
+    k0 += nch;
+  }
+  std::vector<double> h(pop_out || norm_out ? (pop_out ? hist : 0) + (norm_out ? hist : 0) : 0);
+  if (!h.empty())
+    CK(cudaMemcpyAsync(h.data(), f->hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,
+                       c->stream));
+  unsigned st = 0;
+  CK(cudaMemcpyAsync(&st, c->d_status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (st) {
+    CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+    return mpc_fail(MPC_ERR_DEVICE, "kernel status 0x%x in the batched propagation", st);
+  }
+  for (int b = 0; b < B; ++b) {
+    if (pop_out) {
+      const double* x = ct + 2 * ((size_t)b * n + pop_index);
+      pop_out[b * ld] = x[0] * x[0] + x[1] * x[1];
+      for (int k = 1; k <= steps[b]; ++k) pop_out[b * ld + k] = h[b * ld + k];
+    }
+    const double* hn = h.data() + (pop_out ? hist : 0);
+    for (int k = 0; norm_out && k < steps[b]; ++k) norm_out[b * (ld - 1) + k] = hn[b * ld + k];
+  }
+  CK(cudaMemcpyAsync(ct, out, sizeof(double2) * (size_t)B * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return MPC_OK;
+}

@@ -1,0 +1,569 @@
+// flow_batch.cuh -- many pulses on a system whose coupling fits on chip: one
+// persistent cooperative launch for all steps of all pulses, each right-hand
+// side an FP64 tensor-core product (mma.sync m8n8k4 .f64) whose left operand,
+// the coupling, never leaves the registers.
+//
+// Layout.  The CTAs form ng column groups; a group's CTAs together hold every
+// row once, and each group works on its own pulses, in chunks of 8.  A CTA's
+// rows lie in one state block L, so they all couple to the same window
+// (blocks L-1 and L+1).  Its 8 compute warps split the window: warp w takes
+// every 8th group of 4 window rows, and keeps the MT x KT m8k4 fragments of its
+// share of the coupling in registers.  A window element (one pulse, re and im)
+// is one 16-byte load per lane straight into the right operand's fragment
+// layout: lane (k, pulse) of a 4 x 8 tile feeds one m8n8 tile with the real
+// parts and one with the imaginary parts.  So a step of the loop is one load
+// and 2 MT DMMAs, with no shared memory in between; the warps' partial sums
+// meet in shared memory once per item, where one thread per (row, pulse) does
+// the rest of the item in FP64.
+//
+// Why: the stage GEMM (batch_stage.cuh) reloads coupling tiles for every
+// product and leaves most SMs idle below about 128 pulses (90 tiles at 48
+// pulses); here every SM holds its share for the whole run whatever the width,
+// and the chunks hide each other's exchange.
+//
+// Exchange as in resident_flow.cuh: rows are published with 16-byte stores and
+// polled by their readers in buffers preset to kEmpty; a chunk's buffers
+// rotate by step, a helper warp presets them and does the per-pulse control
+// (norms, times, fields, step sizes) from all CTAs' partial sums, redundantly
+// and identically in every CTA.
+//
+// Modes: 0 fixed step (12 Horner products, the reference's semantics),
+// 1 adaptive (13 stages, embedded error, per-pulse step control), 2 the
+// transposed Horner products of the objective gradient.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "batch_types.h"
+#include "dev_util.cuh"
+#include "plan.h"
+#include "resident_flow.cuh"
+#include "rkf78.h"
+
+namespace mpc {
+
+constexpr int CP = 8;               // pulses per chunk
+constexpr int kMaxChunks = 32;      // chunks per column group and launch
+constexpr int kMaxMT = 6;           // 8-row tiles per CTA
+
+struct FbCta {
+  int L, row0, nrows;
+  int grp, idx;      // column group, index within it
+  int cfg;           // which MT x KT instance
+};
+
+struct FbArgs {
+  const double* D;
+  const double* eps;
+  const FbCta* cta;
+  int gp;                 // CTAs per column group
+  int ng;                 // column groups
+  int nch;                // chunks of this launch: chunk c belongs to group c % ng
+  const int* cid;         // [nch][CP] pulse ids (-1: empty slot)
+  const int* csteps;      // [nch] steps of the chunk's longest pulse (descending per group)
+  double2* V;             // [nch][slots][ntot][CP] vectors in flight
+  int slots;
+  double* part;           // [nch][2][gp][2 * CP] norm (and error) partials
+  unsigned long long* ctr;  // [nch] helpers' arrivals
+  unsigned* status;
+  double2* xst;           // [nch][ntot][CP] the step's x
+  const double2* in;      // start states by pulse id, [id][ntot]
+  double2* out;           // final states by pulse id
+  const mpc_pulse* pulse; // by pulse id
+  const double* t0;       // by pulse id
+  const int* nsteps;      // by pulse id
+  const double* Ftab;     // [step][ldf] by pulse id, or null: the pulses' own fields
+  int ldf;
+  double dt;
+  int gauge;
+  int pop_index;
+  long long hist_ld;
+  double* pop_hist;       // [id][hist_ld]
+  double* norm_hist;      // [id][hist_ld]
+  BarrierCfg bc;
+  Geometry g;
+};
+
+__device__ __forceinline__ void dmma884(double* c, double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// What the helper tells the compute warps about a chunk.
+struct FbCtl {
+  double2 nrm[kMaxChunks][CP];   // norm of x and its reciprocal
+  double F[kMaxChunks][CP];      // the step's field
+  double t[kMaxChunks][CP];
+  int id[kMaxChunks][CP];
+  int ns[kMaxChunks][CP];        // the pulse's steps
+  int nst[kMaxChunks];           // the chunk's steps
+  volatile int step[kMaxChunks]; // control is done up to this step
+  volatile int progress;         // (step, chunk) pairs the compute warps finished
+  volatile int hdead, mexit;
+  volatile int mdead[2];         // a wait ran out, by item parity
+};
+
+struct FbView {
+  FlowWin w;
+  int r0;           // first row within block L
+  int nrows, row0, L, nc, grp, idx;
+  long long cpitch; // V elements per chunk
+  long long spitch; // V elements per slot
+};
+
+__device__ __forceinline__ const double2* fb_slot(const FbArgs& a, const FbView& u, int c, int slot) {
+  return a.V + u.cpitch * (c * a.ng + u.grp) + u.spitch * slot;
+}
+
+// ---- one item: the coupling of one chunk's window, summed over the warps ----
+template <int MT, int KT>
+struct FbTile {
+  // Window loads go out in batches, one batch ahead of the DMMAs: single loads
+  // issued a few steps ahead share their scoreboards with the DMMAs, whose
+  // waits then also wait for the loads (400 cycles per step, measured, against
+  // 270 in batches of 3 to 6 and 192 of DMMA).  The rest is L2: all of a
+  // group's CTAs read the same fresh lines at about the same time, at 12 bytes
+  // per cycle and SM in such bursts (27 when the SMs stream apart).  Tried: a
+  // copy ring in shared memory (cp.async) instead of registers (twice as slow:
+  // what is not there yet is sent for again), the coupling in shared memory
+  // and longer batches (+20 to +50 %), separate epilogue warps (+2 %).
+  static constexpr int BD = MT * KT > 60 || KT <= 6 ? 3 : 4;
+  static constexpr int NB = (KT + BD - 1) / BD;
+  double A[MT][KT];
+  double2 b[2][BD];
+  int nj;                      // groups of 4 window rows of this warp
+  int klast, nlo;              // the last lanes' rows are clamped to the window
+  int k0;
+  long long lo, up;            // element offsets of the two blocks' rows
+
+  __device__ __forceinline__ void init(const FbArgs& a, const FbView& u, int warp, int lane) {
+    const int K = u.w.K();
+    nj = max(0, (K - 4 * warp + 4 * FW - 1) / (4 * FW));
+    klast = K - 1;
+    nlo = u.w.nlo;
+    k0 = 4 * warp + (lane & 3);
+    lo = (long long)u.w.lo0 * CP + (lane >> 2);
+    up = (long long)(u.w.up0 - u.w.nlo) * CP + (lane >> 2);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int j = 0; j < KT; ++j) {
+        const int lr = m * 8 + (lane >> 2), k = k0 + 4 * FW * j;
+        A[m][j] = (lr < u.nrows && k < K)
+                      ? flow_coupling(a.g, a.D, a.gauge, u.L, u.r0 + lr, u.w, k)
+                      : 0.0;
+      }
+  }
+  // this lane's element of the warp's j-th group (past the window: its last
+  // row, against a zero coupling)
+  __device__ __forceinline__ const double2* at(const double2* src, int j) const {
+    const int k = min(k0 + 4 * FW * j, klast);
+    return src + (k < nlo ? lo : up) + k * CP;
+  }
+  __device__ __forceinline__ void load(const double2* src, int nb) {
+#pragma unroll
+    for (int i = 0; i < BD; ++i)
+      if (nb * BD + i < KT && nb * BD + i < nj) b[nb & 1][i] = ld_relaxed2(at(src, nb * BD + i));
+  }
+  __device__ __forceinline__ void prefetch(const double2* src) { load(src, 0); }
+  static __device__ __forceinline__ bool missing(double2 v) { return is_empty(v.x) || is_empty(v.y); }
+
+  // acc = coupling x window, polling what is not there yet; the first batch has
+  // been sent for
+  __device__ __forceinline__ void run(const double2* src, double (&acc)[MT][4], volatile int* dead,
+                                      unsigned* status, unsigned long long limit_ns) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[m][v] = 0.0;
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      if (nb * BD >= nj) break;
+      double2* y = b[nb & 1];
+      unsigned long long t0 = 0;
+      for (unsigned it = 0;; ++it) {
+        bool miss = false;
+#pragma unroll
+        for (int i = 0; i < BD; ++i)
+          if (nb * BD + i < KT && nb * BD + i < nj) miss = miss || missing(y[i]);
+        if (!__any_sync(0xffffffffu, miss) || *dead) break;
+#pragma unroll
+        for (int i = 0; i < BD; ++i)
+          if (nb * BD + i < KT && nb * BD + i < nj && missing(y[i]))
+            y[i] = ld_relaxed2(at(src, nb * BD + i));
+        if ((it & 255u) == 255u) {
+          const unsigned long long t = globaltimer_ns();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > limit_ns) {
+            *dead = 1;
+            atomicOr(status, ST_WAIT_TIMEOUT);
+          }
+        }
+      }
+      __syncwarp();
+      if (nb + 1 < NB) load(src, nb + 1);
+#pragma unroll
+      for (int i = 0; i < BD; ++i) {
+        if (nb * BD + i >= KT || nb * BD + i >= nj) continue;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          dmma884(acc[m], A[m][nb * BD + i], y[i].x);
+          dmma884(acc[m] + 2, A[m][nb * BD + i], y[i].y);
+        }
+      }
+    }
+  }
+  // partial sums to red[warp * MT * 64 + row * 8 + pulse]
+  static __device__ __forceinline__ void put(const double (&acc)[MT][4], double2* red, int warp,
+                                             int lane) {
+    double2* r = red + warp * (MT * 64) + (lane >> 2) * 8 + 2 * (lane & 3);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      r[m * 64] = make_double2(acc[m][0], acc[m][2]);
+      r[m * 64 + 1] = make_double2(acc[m][1], acc[m][3]);
+    }
+  }
+};
+
+// The coupling sum of element e, the warps' parts in order.
+template <int MT>
+__device__ __forceinline__ double2 fb_sum(const double2* red, int e) {
+  double2 s[FW];
+#pragma unroll
+  for (int q = 0; q < FW; ++q) s[q] = red[q * (MT * 64) + e];
+  double2 t;
+  t.x = ((s[0].x + s[1].x) + (s[2].x + s[3].x)) + ((s[4].x + s[5].x) + (s[6].x + s[7].x));
+  t.y = ((s[0].y + s[1].y) + (s[2].y + s[3].y)) + ((s[4].y + s[5].y) + (s[6].y + s[7].y));
+  return t;
+}
+
+// M(F) v of one row: e its energy, W its coupling sum.
+__device__ __forceinline__ double2 fb_m(int gauge, double e, double F, double2 v, double2 W) {
+  if (gauge == 0)  // -i (e v + F W)
+    return make_double2(fma(F, W.y, e * v.y), -fma(F, W.x, e * v.x));
+  return make_double2(fma(F, W.x, e * v.y), fma(F, W.y, -e * v.x));  // -i e v + F W
+}
+
+// Waits until the helper is done with chunk c up to `step`; false if the
+// helper gave up (its own waits are bounded).
+__device__ __forceinline__ bool fb_await(FbCtl& ctl, int c, int step) {
+  while (ctl.step[c] < step)
+    if (ctl.hdead || ctl.mexit) return ctl.step[c] >= step;
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// fixed step: slots 2 x 11 Horner vectors by step parity, then 3 x x_{n+1}
+// ---------------------------------------------------------------------------
+constexpr int kFixSlots = 25;
+__device__ __forceinline__ int fix_v(int step, int p) { return (step & 1) * 11 + p; }
+__device__ __forceinline__ int fix_x(int step) { return 22 + (step + 3) % 3; }   // x_{step+1}
+
+// x_step of one element is formed from the unnormalised z; the pulse's
+// population and, at its end, its final state go out.
+__device__ __forceinline__ double2 fix_begin(const FbArgs& a, FbCtl& ctl, int c, int q, int row,
+                                             int step, double2 z) {
+  const double2 x = quot2(z, ctl.nrm[c][q]);
+  const int id = ctl.id[c][q];
+  if (id >= 0 && step <= ctl.ns[c][q]) {
+    if (a.pop_hist && row == a.pop_index && step > 0)
+      a.pop_hist[(long long)id * a.hist_ld + step] =
+          __dadd_rn(__dmul_rn(x.x, x.x), __dmul_rn(x.y, x.y));
+    if (step == ctl.ns[c][q]) a.out[(long long)id * a.g.ntot + row] = x;
+  }
+  return x;
+}
+
+template <int MT, int KT>
+__device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, double2* red,
+                              double (*red8)[CP], int tid) {
+  constexpr int NE = (MT * 64 + FT - 1) / FT;   // elements per thread, of one pulse
+  const int warp = tid >> 5, lane = tid & 31, q = tid & 7;
+  FbTile<MT, KT> tile;
+  tile.init(a, u, warp, lane);
+  const double h = a.dt;
+  const int ne = u.nrows * CP;
+  auto slot = [&](int c, int s) {
+    return a.V + u.cpitch * (c * a.ng + u.grp) + u.spitch * s + (long long)u.row0 * CP;
+  };
+  // the start states, as given
+  for (int c = 0; c < u.nc; ++c)
+    for (int e = tid; e < ne; e += FT) {
+      const int id = ctl.id[c][q];
+      publish(slot(c, fix_x(-1)) + e, id >= 0 ? a.in[(long long)id * a.g.ntot + u.row0 + (e >> 3)]
+                                              : make_double2(0.0, 0.0));
+    }
+  // items: per step, per product, the chunks with steps left (the longest first)
+  int it = 0, act = u.nc;
+  bool primed = false;
+  for (int step = 0;; ++step) {
+    while (act > 0 && ctl.nst[act - 1] <= step) {
+      // the last state of a chunk that has finished
+      const int c = --act;
+      if (!fb_await(ctl, c, step)) ctl.mdead[it & 1] = 1;
+      for (int e = tid; e < ne; e += FT)
+        fix_begin(a, ctl, c, q, u.row0 + (e >> 3), step, __ldcg(slot(c, fix_x(step - 1)) + e));
+    }
+    if (act == 0) return;
+#pragma unroll 1
+    for (int p = 0; p < kFlowProducts; ++p) {
+      const bool last = p == kFlowProducts - 1;
+      const double gm = f_G[11 - p], sc = p == 0 ? f_G[12] : 1.0;
+#pragma unroll 1
+      for (int c = 0; c < act; ++c, ++it) {
+        const int in_slot = p == 0 ? fix_x(step - 1) : fix_v(step, p - 1);
+        const double2* src = fb_slot(a, u, c, in_slot);
+        if (!primed) tile.prefetch(src);
+        double acc[MT][4];
+        tile.run(src, acc, &ctl.mdead[it & 1], a.status, a.bc.wait_ns);
+        // the next item's first loads, where its buffer is known to be preset
+        primed = act > 1;
+        if (primed) {
+          const double2* next = nullptr;
+          if (c + 1 < act)
+            next = fb_slot(a, u, c + 1, in_slot);
+          else if (!last)
+            next = fb_slot(a, u, 0, fix_v(step, p));
+          else if (ctl.nst[0] > step + 1)
+            next = fb_slot(a, u, 0, fix_x(step));
+          primed = next != nullptr;
+          if (primed) tile.prefetch(next);
+        }
+        double2* rb = red + (it & 1) * (FW * MT * 64);
+        tile.put(acc, rb, warp, lane);
+        // this thread's own elements of x and of the product's input
+        double2 xo[NE], vo[NE];
+        const double2* own = slot(c, in_slot);
+        double2* xs = a.xst + ((long long)(c * a.ng + u.grp) * a.g.ntot + u.row0) * CP;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e < ne) {
+            vo[i] = __ldcg(own + e);
+            if (p > 0) xo[i] = xs[e];
+          }
+        }
+        named_bar_sync(kBarMain, FT);
+        if (ctl.mdead[it & 1]) return;
+        if (p == 0 && !fb_await(ctl, c, step)) ctl.mdead[(it + 1) & 1] = 1;
+        const double F = ctl.F[c][q];
+        double2* dst = slot(c, last ? fix_x(step) : fix_v(step, p));
+        double nsq = 0.0;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e >= ne) continue;
+          const int row = u.row0 + (e >> 3);
+          double2 W = fb_sum<MT>(rb, e), x = xo[i], v = vo[i];
+          if (p == 0) {
+            x = fix_begin(a, ctl, c, q, row, step, v);
+            xs[e] = x;
+            v = make_double2(sc * x.x, sc * x.y);   // v_12 = G_12 x
+            W = quot2(W, ctl.nrm[c][q]);
+            W.x *= sc;
+            W.y *= sc;
+          }
+          const double2 m = fb_m(a.gauge, a.eps[row], F, v, W);
+          const double2 o = make_double2(fma(h, m.x, gm * x.x), fma(h, m.y, gm * x.y));
+          publish(dst + e, o);
+          nsq += fma(o.x, o.x, o.y * o.y);
+        }
+        if (last) {
+          // the CTA's norm partial per pulse: a thread's rows, the lanes of its
+          // pulse, the warps in order
+          nsq += __shfl_xor_sync(0xffffffffu, nsq, 8);
+          nsq += __shfl_xor_sync(0xffffffffu, nsq, 16);
+          if (lane < CP) red8[warp][lane] = nsq;
+          named_bar_sync(kBarMain, FT);
+          if (tid < CP) {
+            double t = red8[0][tid];
+#pragma unroll
+            for (int k = 1; k < FW; ++k) t += red8[k][tid];
+            st_relaxed1(a.part + (((long long)(c * a.ng + u.grp) * 2 + (step & 1)) * a.gp + u.idx) *
+                                     (2 * CP) + tid,
+                        canonical(t));
+          }
+          __syncwarp();
+          if (tid == 0) ctl.progress = ctl.progress + 1;
+        }
+      }
+    }
+  }
+}
+
+// Per chunk and step: the norms from all CTAs' partials, the pulses' times and
+// next fields, the presets.  One warp; lane = (quarter of the CTAs, pulse).
+__device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, int lane) {
+  const int q = lane & 7;
+  auto field = [&](int c, int step) {
+    const int id = ctl.id[c][q];
+    if (id < 0 || step >= ctl.ns[c][q]) return 0.0;
+    if (a.Ftab) return a.Ftab[(long long)step * a.ldf + id];
+    return dev_field(a.pulse[id], ctl.t[c][q] + a.dt);
+  };
+  for (int c = 0; c < u.nc; ++c) {
+    if (lane < CP) {
+      ctl.nrm[c][q] = make_double2(1.0, 1.0);
+      ctl.t[c][q] = ctl.id[c][q] >= 0 && a.t0 ? a.t0[ctl.id[c][q]] : 0.0;
+      ctl.F[c][q] = field(c, 0);
+    }
+    __syncwarp();
+    __threadfence_block();
+    if (lane == 0) ctl.step[c] = 0;
+  }
+  int events = 0;
+  for (int n = 0;; ++n) {   // event n: step n of a chunk is complete
+    bool any = false;
+    for (int c = 0; c < u.nc && ctl.nst[c] > n; ++c) {
+      any = true;
+      ++events;
+      bool ok = true;
+      while (ok && ctl.progress < events) ok = ctl.mexit == 0;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      const int gc = c * a.ng + u.grp;
+      if (n > 0) {   // everyone's presets of event n - 1 are made
+        if (lane == 0) {
+          unsigned long long v = 0, t0 = 0;
+          for (unsigned i = 0;; ++i) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a.ctr + gc) : "memory");
+            if (v >= (unsigned long long)n * a.gp + a.bc.skew) break;
+            if ((i & 1023u) == 1023u) {
+              const unsigned long long t = globaltimer_ns();
+              if (t0 == 0) t0 = t;
+              if (t - t0 > a.bc.wait_ns) {
+                ok = false;
+                break;
+              }
+            }
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+      }
+      double sum = 0.0;
+      const double* pp = a.part + ((long long)gc * 2 + (n & 1)) * a.gp * (2 * CP);
+      for (int b0 = lane >> 3; ok && b0 < a.gp; b0 += 32) {
+        double v[8];
+        unsigned long long t0 = 0;
+        for (unsigned i = 0;; ++i) {
+          bool ready = true;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            v[j] = b0 + 4 * j < a.gp ? ld_relaxed1(pp + (b0 + 4 * j) * (2 * CP) + q) : 0.0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ready = ready && !is_empty(v[j]);
+          if (ready) break;
+          if ((i & 255u) == 255u) {
+            const unsigned long long t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > a.bc.wait_ns) {
+              ok = false;
+              break;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum += v[j];
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) {
+          atomicOr(a.status, ST_WAIT_TIMEOUT);
+          ctl.hdead = 1;
+        }
+        return;
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      if (lane < CP) {
+        const int id = ctl.id[c][q];
+        double nrm = sqrt(sum);
+        if (id < 0) nrm = 1.0;
+        if (id >= 0 && n < ctl.ns[c][q]) {
+          ctl.t[c][q] += a.dt;
+          if (u.idx == 0) {
+            if (a.norm_hist) a.norm_hist[(long long)id * a.hist_ld + n] = nrm;
+            if (!(nrm > 0.0) || !isfinite(nrm)) atomicOr(a.status, ST_NONFINITE);
+          }
+        }
+        ctl.nrm[c][q] = make_double2(nrm, 1.0 / nrm);
+        ctl.F[c][q] = field(c, n + 1);
+        st_relaxed1(a.part + (((long long)gc * 2 + ((n + 1) & 1)) * a.gp + u.idx) * (2 * CP) + q,
+                    __longlong_as_double((long long)kEmpty));
+      }
+      __syncwarp();
+      __threadfence_block();
+      if (lane == 0) ctl.step[c] = n + 1;
+      // every CTA is past step n of this chunk: its Horner vectors, and x_n
+      double2* base = a.V + u.cpitch * gc + (long long)u.row0 * CP;
+      const int ne = u.nrows * CP;
+      for (int s = 0; s <= 11; ++s) {
+        double2* d = base + u.spitch * (s < 11 ? fix_v(n, s) : fix_x(n - 1));
+        for (int e = lane; e < ne; e += 32) st_relaxed2(d + e, empty2());
+      }
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(a.ctr + gc), "l"(1ull)
+                     : "memory");
+    }
+    if (!any) return;
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constant__ FbArgs a) {
+  extern __shared__ __align__(16) unsigned char bsm[];
+  const FbCta me = a.cta[blockIdx.x];
+  FbCtl& ctl = *reinterpret_cast<FbCtl*>(bsm);
+  double2* red = reinterpret_cast<double2*>(bsm + (sizeof(FbCtl) + 15) / 16 * 16);
+  __shared__ double red8[FW][CP];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  FbView u;
+  u.w = flow_window(a.g, me.L);
+  u.L = me.L;
+  u.row0 = me.row0;
+  u.nrows = me.nrows;
+  u.r0 = me.row0 - a.g.state_off[me.L];
+  u.grp = me.grp;
+  u.idx = me.idx;
+  u.nc = (a.nch - me.grp + a.ng - 1) / a.ng;
+  u.spitch = (long long)a.g.ntot * CP;
+  u.cpitch = u.spitch * a.slots;
+  for (int i = tid; i < u.nc * CP; i += FTHREADS) {
+    const int c = i / CP, q = i % CP, id = a.cid[(c * a.ng + me.grp) * CP + q];
+    ctl.id[c][q] = id;
+    ctl.ns[c][q] = id >= 0 && a.nsteps ? a.nsteps[id] : 0;
+    if (q == 0) {
+      ctl.nst[c] = a.csteps[c * a.ng + me.grp];
+      ctl.step[c] = -1;
+    }
+  }
+  if (tid == 0) {
+    ctl.progress = 0;
+    ctl.hdead = ctl.mexit = 0;
+    ctl.mdead[0] = ctl.mdead[1] = 0;
+  }
+  __syncthreads();
+#define FB_CONFIGS(X) \
+  X(0, 1, 6) X(1, 2, 6) X(2, 4, 6) X(3, 2, 10) X(4, 4, 10) X(5, 6, 10) X(6, 2, 13) X(7, 5, 13) \
+  X(8, 2, 19) X(9, 3, 19) X(10, 2, 25) X(11, 3, 25)
+  if (warp >= FW) {
+    regs_dec<40>();
+    if (warp == FW) fb_fixed_helper(a, ctl, u, lane);
+    return;
+  }
+  regs_inc<232>();
+#define FB_RUN(I, MT, KT) \
+  case I: fb_fixed_main<MT, KT>(a, ctl, u, red, red8, tid); break;
+  switch (me.cfg) { FB_CONFIGS(FB_RUN) }
+#undef FB_RUN
+  if (tid == 0) ctl.mexit = 1;
+}
+
+// Shared memory of a CTA: control and two buffers of partial sums.
+inline size_t flowb_smem() {
+  return (sizeof(FbCtl) + 15) / 16 * 16 + sizeof(double2) * 2 * FW * kMaxMT * 64;
+}
+
+}  // namespace mpc

@@ -1,0 +1,13 @@
+// flow_batch.h -- the persistent batched propagation for systems whose
+// coupling fits on chip (flow_batch.cu).
+#pragma once
+#include <cstddef>
+
+#include "ctx.h"
+
+bool mpc_flowb_setup(mpc_ctx* c);   // usable for this system
+bool mpc_flowb_wanted(mpc_ctx* c, int B);   // and the faster path for B pulses
+void mpc_flowb_free(mpc_ctx* c);
+int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
+                      const int* steps, int pop_index, double* ct, double* pop_out,
+                      double* norm_out, int max_steps);

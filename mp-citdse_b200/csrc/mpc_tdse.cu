@@ -16,6 +16,7 @@
 #include "../../include/mpc_tdse.h"
 #include "combine.cuh"
 #include "ctx.h"
+#include "flow_batch.h"
 #include "plan.h"
 #include "rhs_stream.cuh"
 #include "rkf78.h"
@@ -686,6 +687,7 @@ int mpc_ctx_destroy(mpc_ctx* c) {
   mpc_resident_free(c);
   mpc_batch_res_free(c);
   mpc_badj_free(c);
+  mpc_flowb_free(c);
   free_all(c);
   for (auto& v : c->ev)
     for (auto& pr : v) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }

@@ -42,6 +42,45 @@ const FlowKernel kAdjoint[] = {
 #undef FWD
 #undef ADJ
 
+// dJ/dF_n = sum over the CTAs' partials of step n: one warp per step, lanes
+// striding, then a fixed xor tree.
+__global__ void k_flow_fbar(const double* fpart, int steps, int np, double* fbar) {
+  const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (n >= steps) return;
+  double t = 0.0;
+  for (int p = lane; p < np; p += 32) t += fpart[(long long)n * np + p];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) fbar[n] = t;
+}
+
+// lambda_N = (1 - x x^T) dJ/dx_N, x = x_N (unit norm): yield -> 2 x on the
+// states at or above the threshold, target -> 2 x_t.  One CTA; the projection
+// is the last step's normalisation adjoint.
+__global__ void k_flow_seed(const double2* x, const double* eps, double2* lam, int target,
+                            double thr, int ntot) {
+  __shared__ double sh[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto seed = [&](int i) {
+    const double2 v = x[i];
+    const bool on = target < 0 ? eps[i] >= thr : i == target;
+    return on ? make_double2(2.0 * v.x, 2.0 * v.y) : make_double2(0.0, 0.0);
+  };
+  double d = 0.0;
+  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
+    const double2 v = x[i], l = seed(i);
+    d += fma(v.x, l.x, v.y * l.y);
+  }
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  if (lane == 0) sh[warp] = d;
+  __syncthreads();
+  d = 0.0;
+  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) d += sh[q];
+  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
+    const double2 v = x[i], l = seed(i);
+    lam[i] = make_double2(fma(-d, v.x, l.x), fma(-d, v.y, l.y));
+  }
+}
+
 constexpr size_t kFlowStatic = 256;   // the kernels' static shared memory, rounded up
 
 int window_len(const Geometry& g, int L) {
@@ -138,8 +177,7 @@ bool plan_kernel(const Geometry& g, const FlowKernel (&list)[N], int NC, size_t 
     size_t smem = 0;
     if (!fit_kernel(g, k, NC, limit, ctas, &smem)) continue;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
+    if (!mpc_allow_smem(k.fn, (int)limit) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, FTHREADS, smem) !=
             cudaSuccess ||
         per_sm < 1) {
@@ -175,6 +213,17 @@ struct mpc_resident_state {
   double* fpart = nullptr;
   size_t fpart_n = 0;
 };
+
+// All the dynamic shared memory a block may have: the attribute belongs to the
+// function, so a context must not set it to its own, smaller need.
+bool mpc_allow_smem(const void* fn, int optin) {
+  cudaFuncAttributes at{};
+  const bool ok = cudaFuncGetAttributes(&at, fn) == cudaSuccess &&
+                  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       optin - (int)at.sharedSizeBytes) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
 
 // Sets up the resident path if the system fits; returns true when usable.
 bool mpc_resident_setup(mpc_ctx* c) {

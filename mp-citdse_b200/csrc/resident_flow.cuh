@@ -72,7 +72,7 @@ struct FlowCta {
   int cg;       // column groups (1, 2, 4, 8); FW / cg row groups
 };
 
-__constant__ double f_G[13];
+static __constant__ double f_G[13];   // the stability polynomial's coefficients
 
 __device__ __forceinline__ double2 ld_relaxed2(const double2* p) {
   double2 v;
@@ -868,45 +868,6 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_adjoint(const __grid_const
     }
   }
   if (isrow) a.lam[row] = lam;
-}
-
-// dJ/dF_n = sum over the CTAs' partials of step n: one warp per step, lanes
-// striding, then a fixed xor tree.
-__global__ void k_flow_fbar(const double* fpart, int steps, int np, double* fbar) {
-  const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (n >= steps) return;
-  double t = 0.0;
-  for (int p = lane; p < np; p += 32) t += fpart[(long long)n * np + p];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0) fbar[n] = t;
-}
-
-// lambda_N = (1 - x x^T) dJ/dx_N, x = x_N (unit norm): yield -> 2 x on the
-// states at or above the threshold, target -> 2 x_t.  One CTA; the projection
-// is the last step's normalisation adjoint.
-__global__ void k_flow_seed(const double2* x, const double* eps, double2* lam, int target,
-                            double thr, int ntot) {
-  __shared__ double sh[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto seed = [&](int i) {
-    const double2 v = x[i];
-    const bool on = target < 0 ? eps[i] >= thr : i == target;
-    return on ? make_double2(2.0 * v.x, 2.0 * v.y) : make_double2(0.0, 0.0);
-  };
-  double d = 0.0;
-  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
-    const double2 v = x[i], l = seed(i);
-    d += fma(v.x, l.x, v.y * l.y);
-  }
-  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-  if (lane == 0) sh[warp] = d;
-  __syncthreads();
-  d = 0.0;
-  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) d += sh[q];
-  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
-    const double2 v = x[i], l = seed(i);
-    lam[i] = make_double2(fma(-d, v.x, l.x), fma(-d, v.y, l.y));
-  }
 }
 
 }  // namespace mpc

@@ -1,0 +1,55 @@
+"""The persistent batched kernels (systems whose coupling fits on chip) at the
+sizes where their layout can go wrong: one-row blocks, blocks much longer or
+shorter than their neighbours, every row tile, pulse counts around the chunks
+of 8 and the column groups, pulses without steps, single steps.
+
+Each pulse against the single-pulse path (or, for adaptive steps, the CPU
+oracle).  A step is 12 products whose sums round at 1e-16 of |h M v| <= 2.4 |v|
+in two different orders, so n steps agree within n x 13 x 2.4 x ~50 eps:
+3e-13 per step in any coefficient of a unit-norm state, twice that in norms
+and populations.
+"""
+import numpy as np
+import pytest
+
+import mpc_tdse
+from mpc_tdse.systems import random_system
+
+pytestmark = pytest.mark.gpu
+
+SYSTEMS = [[1, 1], [1, 7, 1, 2], [60, 70, 50], [97] * 5, [201] * 8, [292] * 6, [33] * 16,
+           [388, 387, 386, 385, 384, 383, 382, 381, 380], [5, 500, 7]]
+
+
+def _case(n, gauge, B):
+    s = random_system(n, gauge=gauge, seed=len(n), e_max=8.0, d_scale=0.3)
+    rng = np.random.default_rng(B)
+    pulses = []
+    for b in range(B):
+        Io, w = mpc_tdse.to_au(2e14 * (1 + b % 5), 4.0 + 0.1 * (b % 7))
+        pulses.append(mpc_tdse.pulse_setup("gaussian" if b % 3 == 2 else "sine", gauge, Io, w,
+                                           0.1 * b, 2, mpc_tdse.period(w, 2)))
+    X = rng.standard_normal((B, s.ntot)) + 1j * rng.standard_normal((B, s.ntot))
+    return s, pulses, X / np.linalg.norm(X, axis=1, keepdims=True)
+
+
+@pytest.mark.parametrize("gauge", ["l", "v"])
+@pytest.mark.parametrize("B", [1, 7, 8, 9, 35])
+@pytest.mark.parametrize("n", SYSTEMS, ids=lambda n: f"{len(n)}x{max(n)}")
+def test_fixed_steps_match_single_pulse(n, B, gauge):
+    s, pulses, X = _case(n, gauge, B)
+    steps = np.array([(5 * b + 3) % 7 for b in range(B)])   # 0 to 6, one of them 0 from B = 7
+    t0 = 0.3 * np.arange(B)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        Y, pop, nrm = ctx.batch_advance(pulses, t0, 0.1, steps, X, pop_index=s.ntot - 1,
+                                        history=True)
+        for b in range(B):
+            k = int(steps[b])
+            if k == 0:
+                assert np.array_equal(Y[b], X[b])
+                continue
+            ct, p1, _, n1 = ctx.propagate(pulses[b], t0[b], 0.1, k, X[b], pop_index=s.ntot - 1)
+            assert np.max(np.abs(Y[b] - ct)) < 3e-13 * k, b
+            assert np.max(np.abs(pop[b, :k + 1] - p1)) < 6e-13 * k, b
+            assert np.max(np.abs(nrm[b, :k] - n1)) < 6e-13 * k, b
+            assert np.all(np.isnan(nrm[b, k:])) and np.all(np.isnan(pop[b, k + 1:]))
