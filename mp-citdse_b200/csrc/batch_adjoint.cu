@@ -26,6 +26,7 @@
 #include "batch_stage.cuh"
 #include "batch_types.h"
 #include "ctx.h"
+#include "flow_batch.h"
 
 using namespace mpc;
 
@@ -142,6 +143,7 @@ struct mpc_badj_state {
   double dt = 0.0;
   std::vector<double> T, u, tn;
   bool have_forward = false;
+  bool flow = false;         // the last forward ran on the persistent kernels (flow_batch.cu)
   // device buffers ([n][ldc] complex unless noted)
   double2* ckpts = nullptr;  // [nseg + 1]
   double2* segX = nullptr;   // [ckpt + 1]
@@ -362,11 +364,19 @@ int mpc_batch_objective(mpc_ctx* c, int B, const mpc_pulse* pulses, int K, const
                     dt * c->eps_max);
   CK(cudaSetDevice(c->device));
   int rc;
-  if ((rc = stage_setup(c->device))) return rc;
-  if (ckpt_every <= 0 && (rc = auto_ckpt(c, B, steps, &ckpt_every))) return rc;
-  if ((rc = ensure_badj(c, B, steps, ckpt_every))) return rc;
+  const bool flow = mpc_flowb_objective_wanted(c, B);
+  if (!c->badj) c->badj = new mpc_badj_state();
   mpc_badj_state* a = c->badj;
+  if (flow) {
+    a->have_forward = false;
+    if (ckpt_every <= 0 && (rc = mpc_flowb_auto_ckpt(c, B, steps, &ckpt_every))) return rc;
+  } else {
+    if ((rc = stage_setup(c->device))) return rc;
+    if (ckpt_every <= 0 && (rc = auto_ckpt(c, B, steps, &ckpt_every))) return rc;
+    if ((rc = ensure_badj(c, B, steps, ckpt_every))) return rc;
+  }
   a->have_forward = false;
+  a->flow = flow;
   a->B = B;
   a->steps = steps;
   a->ckpt = ckpt_every;
@@ -381,7 +391,7 @@ int mpc_batch_objective(mpc_ctx* c, int B, const mpc_pulse* pulses, int K, const
     std::copy(u, u + (size_t)B * a->K, a->u.begin());
   }
   // field table, t accumulated as the reference's loop does (t += dt)
-  const int ldc = a->ldc, n = c->g.ntot;
+  const int ldc = flow ? B : a->ldc, n = c->g.ntot;
   std::vector<double> F((size_t)steps * ldc, 0.0);
   a->tn.resize(steps);
   double t = t0;
@@ -396,6 +406,25 @@ int mpc_batch_objective(mpc_ctx* c, int B, const mpc_pulse* pulses, int K, const
                 : 0.0);
     }
     t += dt;
+  }
+  if (flow) {
+    std::vector<double2> xN((size_t)n * B);
+    std::vector<double> eps(n);
+    CK(cudaMemcpyAsync(eps.data(), c->d_eps, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    if ((rc = mpc_flowb_objective(c, B, F.data(), dt, steps, ckpt_every, ct0, xN.data()))) return rc;
+    for (int b = 0; b < B; ++b) {
+      const double2* x = xN.data() + (size_t)b * n;
+      double y = 0.0;
+      if (target < 0) {
+        for (int i = 0; i < n; ++i)
+          if (eps[i] >= c->yield_thr) y += x[i].x * x[i].x + x[i].y * x[i].y;
+      } else {
+        y = x[target].x * x[target].x + x[target].y * x[target].y;
+      }
+      J[b] = y;
+    }
+    a->have_forward = true;
+    return MPC_OK;
   }
   std::vector<double> hv(ldc, dt);
   CK(cudaMemcpyAsync(a->Ftab, F.data(), sizeof(double) * F.size(), cudaMemcpyHostToDevice,
@@ -460,7 +489,9 @@ int mpc_batch_objective_info(mpc_ctx* c, int* ckpt_every, int* segments, double*
   const mpc_badj_state* a = c->badj;
   if (ckpt_every) *ckpt_every = a->ckpt;
   if (segments) *segments = a->nseg;
-  if (device_bytes) *device_bytes = (double)badj_bytes(c, a->B, a->steps, a->ckpt);
+  if (device_bytes)
+    *device_bytes = (double)(a->flow ? mpc_flowb_objective_bytes(c, a->B, a->steps, a->ckpt)
+                                     : badj_bytes(c, a->B, a->steps, a->ckpt));
   return MPC_OK;
 }
 
@@ -471,63 +502,68 @@ int mpc_batch_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
                                  "mpc_batch_objective");
   CK(cudaSetDevice(c->device));
   mpc_badj_state* a = c->badj;
-  const int B = a->B, ldc = a->ldc, n = c->g.ntot, steps = a->steps, ckpt = a->ckpt;
+  const int B = a->B, ldc = a->flow ? a->B : a->ldc, n = c->g.ntot, steps = a->steps,
+            ckpt = a->ckpt;
   const size_t slab = (size_t)n * ldc;
   const int eb = blocks_for((long long)n * B, 256);
   int rc;
-  k_fb_seed<<<eb, 256, 0, c->stream>>>(a->ckpts + slab * a->nseg, c->d_eps, a->KB[1], a->target,
-                                       c->yield_thr, n, B, ldc);
-  CK(cudaGetLastError());
-  ++c->launches;
-  const double hb12 = a->dt * rkf78::B8[kNumStages - 1];
-  for (int seg = a->nseg - 1; seg >= 0; --seg) {
-    const int n0 = seg * ckpt;
-    const int len = std::min(ckpt, steps - n0);
-    // recompute the segment (the last one is still resident from the
-    // forward pass): states, stage inputs and norms
-    if (seg < a->nseg - 1) {
-      CK(cudaMemcpyAsync(a->segX, a->ckpts + slab * seg, sizeof(double2) * slab,
-                         cudaMemcpyDeviceToDevice, c->stream));
-      for (int j = 0; j < len; ++j)
-        if ((rc = fb_step(c, n0 + j, a->segX + slab * j, a->segY + slab * 12 * (size_t)j,
-                          a->segX + slab * (j + 1), a->segN + (size_t)j * ldc)))
-          return rc;
-    }
-    // walk back through it
-    for (int j = len - 1; j >= 0; --j) {
-      const int stp = n0 + j;
-      const double2* x1 = a->segX + slab * (j + 1);
-      {
-        ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
-        CK(mpc_launch_pdl(k_fb_dot, dim3(a->nchunk, blocks_for(B, 64)), dim3(64), 0, c->stream,
-                          x1, (const double2*)a->KB[1], a->dpart, n, B, ldc));
-        CK(mpc_launch_pdl(k_fb_colsum, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
-                          (const double*)a->dpart, a->nchunk, ldc, B, a->dsum));
-        CK(mpc_launch_pdl(k_fb_zbar, dim3(eb), dim3(256), 0, c->stream, (const double2*)a->KB[1],
-                          x1, (const double*)a->dsum, (const double*)(a->segN + (size_t)j * ldc),
-                          a->Zbar, a->KB[0], hb12, n, B, ldc));
-        c->launches += 3;
-      }
-      for (int s = kNumStages - 1; s >= 0; --s) {
-        StageArgs st = fb_args(c, s, stp);
-        st.Yin = a->KB[(kNumStages - 1 - s) & 1];
-        st.Yout = a->KB[(kNumStages - s) & 1];
-        st.Ys = (s == 0) ? a->segX + slab * j : a->segY + slab * (12 * (size_t)j + (s - 1));
-        st.Zbar = a->Zbar;
-        if ((rc = fb_launch<1>(c, st))) return rc;
-      }
-      {
-        ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
-        CK(mpc_launch_pdl(k_fb_fbar, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
-                          (const double*)a->fpart, a->nrt, ldc, B, a->fbar + (size_t)stp * ldc));
-        ++c->launches;
-      }
-    }
-  }
   std::vector<double> fb((size_t)steps * ldc);
-  CK(cudaMemcpyAsync(fb.data(), a->fbar, sizeof(double) * fb.size(), cudaMemcpyDeviceToHost,
-                     c->stream));
-  if ((rc = check_device_status(c, "batched adjoint pass"))) return rc;
+  if (a->flow) {
+    if ((rc = mpc_flowb_objective_backward(c, a->target, fb.data()))) return rc;
+  } else {
+    k_fb_seed<<<eb, 256, 0, c->stream>>>(a->ckpts + slab * a->nseg, c->d_eps, a->KB[1], a->target,
+                                         c->yield_thr, n, B, ldc);
+    CK(cudaGetLastError());
+    ++c->launches;
+    const double hb12 = a->dt * rkf78::B8[kNumStages - 1];
+    for (int seg = a->nseg - 1; seg >= 0; --seg) {
+      const int n0 = seg * ckpt;
+      const int len = std::min(ckpt, steps - n0);
+      // recompute the segment (the last one is still resident from the
+      // forward pass): states, stage inputs and norms
+      if (seg < a->nseg - 1) {
+        CK(cudaMemcpyAsync(a->segX, a->ckpts + slab * seg, sizeof(double2) * slab,
+                           cudaMemcpyDeviceToDevice, c->stream));
+        for (int j = 0; j < len; ++j)
+          if ((rc = fb_step(c, n0 + j, a->segX + slab * j, a->segY + slab * 12 * (size_t)j,
+                            a->segX + slab * (j + 1), a->segN + (size_t)j * ldc)))
+            return rc;
+      }
+      // walk back through it
+      for (int j = len - 1; j >= 0; --j) {
+        const int stp = n0 + j;
+        const double2* x1 = a->segX + slab * (j + 1);
+        {
+          ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
+          CK(mpc_launch_pdl(k_fb_dot, dim3(a->nchunk, blocks_for(B, 64)), dim3(64), 0, c->stream,
+                            x1, (const double2*)a->KB[1], a->dpart, n, B, ldc));
+          CK(mpc_launch_pdl(k_fb_colsum, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
+                            (const double*)a->dpart, a->nchunk, ldc, B, a->dsum));
+          CK(mpc_launch_pdl(k_fb_zbar, dim3(eb), dim3(256), 0, c->stream, (const double2*)a->KB[1],
+                            x1, (const double*)a->dsum, (const double*)(a->segN + (size_t)j * ldc),
+                            a->Zbar, a->KB[0], hb12, n, B, ldc));
+          c->launches += 3;
+        }
+        for (int s = kNumStages - 1; s >= 0; --s) {
+          StageArgs st = fb_args(c, s, stp);
+          st.Yin = a->KB[(kNumStages - 1 - s) & 1];
+          st.Yout = a->KB[(kNumStages - s) & 1];
+          st.Ys = (s == 0) ? a->segX + slab * j : a->segY + slab * (12 * (size_t)j + (s - 1));
+          st.Zbar = a->Zbar;
+          if ((rc = fb_launch<1>(c, st))) return rc;
+        }
+        {
+          ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
+          CK(mpc_launch_pdl(k_fb_fbar, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
+                            (const double*)a->fpart, a->nrt, ldc, B, a->fbar + (size_t)stp * ldc));
+          ++c->launches;
+        }
+      }
+    }
+    CK(cudaMemcpyAsync(fb.data(), a->fbar, sizeof(double) * fb.size(), cudaMemcpyDeviceToHost,
+                       c->stream));
+    if ((rc = check_device_status(c, "batched adjoint pass"))) return rc;
+  }
   if (dJdF)
     for (int b = 0; b < B; ++b)
       for (int st = 0; st < steps; ++st) dJdF[(size_t)b * steps + st] = fb[(size_t)st * ldc + b];

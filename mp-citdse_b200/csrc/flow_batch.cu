@@ -151,6 +151,31 @@ struct mpc_flowb_state {
   size_t t0_n = 0;
   double* hist = nullptr;    // population and norm histories
   size_t hist_n = 0;
+  // the batched objective's last forward pass (kept for its backward pass, so
+  // in buffers of its own)
+  int oB = 0, osteps = 0, ockpt = 0, ong = 0, onch = 0;
+  bool okept = false;        // seg_v holds the last segment
+  double odt = 0.0;
+  int* oint = nullptr;
+  size_t oint_n = 0;
+  double2* oio = nullptr;    // start states, x_N [B][n]
+  size_t oio_n = 0;
+  double* oF = nullptr;      // fields [steps][B]
+  size_t oF_n = 0;
+  double* onorm = nullptr;   // [B][steps]
+  size_t onorm_n = 0;
+  double2* ockp = nullptr;   // checkpoints
+  size_t ockp_n = 0;
+  double2* oseg = nullptr;   // a segment's vectors
+  size_t oseg_n = 0;
+  double2* olam = nullptr;   // lambda, then the sums of G_m vbar_m
+  size_t olam_n = 0;
+  double* ofs = nullptr;
+  size_t ofs_n = 0;
+  double* ofp = nullptr;     // dJ/dF partials of a segment
+  size_t ofp_n = 0;
+  double* ofb = nullptr;     // dJ/dF [steps][B]
+  size_t ofb_n = 0;
 };
 
 bool mpc_flowb_setup(mpc_ctx* c) {
@@ -179,7 +204,11 @@ bool mpc_flowb_setup(mpc_ctx* c) {
       }
     int per_sm = 0;
     if (!mpc_allow_smem((const void*)&k_flow_batch<0>, optin) ||
+        !mpc_allow_smem((const void*)&k_flow_batch<2>, optin) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flow_batch<0>, FTHREADS,
+                                                      flowb_smem()) != cudaSuccess ||
+        per_sm < 1 ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flow_batch<2>, FTHREADS,
                                                       flowb_smem()) != cudaSuccess ||
         per_sm < 1 || cudaMalloc(&g.ctas, sizeof(FbCta) * all.size()) != cudaSuccess ||
         cudaMemcpy(g.ctas, all.data(), sizeof(FbCta) * all.size(), cudaMemcpyHostToDevice) !=
@@ -206,6 +235,16 @@ void mpc_flowb_free(mpc_ctx* c) {
   cudaFree(f->pulse);
   cudaFree(f->t0);
   cudaFree(f->hist);
+  cudaFree(f->oint);
+  cudaFree(f->oio);
+  cudaFree(f->oF);
+  cudaFree(f->onorm);
+  cudaFree(f->ockp);
+  cudaFree(f->oseg);
+  cudaFree(f->olam);
+  cudaFree(f->ofs);
+  cudaFree(f->ofp);
+  cudaFree(f->ofb);
   delete f;
   c->flowb = nullptr;
 }
@@ -228,6 +267,258 @@ int pick_groups(const mpc_flowb_state* f, int nch) {
 }
 
 }  // namespace
+
+namespace {
+
+// One launch of nch chunks on ng column groups, its work space preset.
+int launch(mpc_ctx* c, FbArgs& a, int ng, int nch, int slots, const void* kernel) {
+  mpc_flowb_state* f = c->flowb;
+  const Group& grp = f->grp[ng];
+  const size_t n = c->g.ntot;
+  const size_t vn = (size_t)nch * slots * n * CP, pn = (size_t)nch * 2 * grp.gp * 2 * CP;
+  int rc;
+  if ((rc = grow(&f->V, &f->V_n, vn)) || (rc = grow(&f->part, &f->part_n, pn)) ||
+      (rc = grow(&f->ctr, &f->ctr_n, (size_t)nch)) || (rc = grow(&f->xst, &f->xst_n, nch * n * CP)))
+    return rc;
+  CK(cudaMemsetAsync(f->V, 0xff, sizeof(double2) * vn, c->stream));
+  CK(cudaMemsetAsync(f->part, 0xff, sizeof(double) * pn, c->stream));
+  CK(cudaMemsetAsync(f->ctr, 0, sizeof(unsigned long long) * nch, c->stream));
+  a.D = c->d_D;
+  a.eps = c->d_eps;
+  a.slots = slots;
+  a.status = c->d_status;
+  a.gauge = (c->gauge == 'l') ? 0 : 1;
+  a.g = c->g;
+  a.cta = grp.ctas;
+  a.gp = grp.gp;
+  a.ng = ng;
+  a.nch = nch;
+  a.V = f->V;
+  a.part = f->part;
+  a.ctr = f->ctr;
+  a.xst = f->xst;
+  a.bc = mpc_barrier_cfg(c);
+  void* args[] = {&a};
+  ProfScope ps(c, MPC_KERNEL_BATCH_STAGE);
+  CK(cudaLaunchCooperativeKernel(kernel, dim3(ng * grp.gp), dim3(FTHREADS), args, flowb_smem(),
+                                 c->stream));
+  return MPC_OK;
+}
+
+// lambda_N of every pulse, projected as k_flow_seed does (one CTA per pulse).
+__global__ void k_fb_seed(const int* cid, const double2* x, const double* eps, double2* lam,
+                          int target, double thr, int ntot) {
+  const int gc = blockIdx.x / CP, q = blockIdx.x % CP, id = cid[blockIdx.x];
+  __shared__ double sh[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double2* xp = x + (long long)max(id, 0) * ntot;
+  auto seed = [&](int i) {
+    const bool on = id >= 0 && (target < 0 ? eps[i] >= thr : i == target);
+    return on ? make_double2(2.0 * xp[i].x, 2.0 * xp[i].y) : make_double2(0.0, 0.0);
+  };
+  double d = 0.0;
+  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
+    const double2 v = xp[i], l = seed(i);
+    d += fma(v.x, l.x, v.y * l.y);
+  }
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  if (lane == 0) sh[warp] = d;
+  __syncthreads();
+  d = 0.0;
+  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) d += sh[k];
+  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
+    double2 l = make_double2(0.0, 0.0);
+    if (id >= 0) {
+      const double2 v = xp[i], s = seed(i);
+      l = make_double2(fma(-d, v.x, s.x), fma(-d, v.y, s.y));
+    }
+    lam[((long long)gc * ntot + i) * CP + q] = l;
+  }
+}
+
+// dJ/dF_n per pulse from the CTAs' partials: a warp per step and chunk.
+__global__ void k_fb_fbar(const double* fpart, const int* cid, int len, int nch, int gp,
+                          double* fbar, int B) {
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= len * nch) return;
+  const int n = w / nch, gc = w % nch, q = lane & 7;
+  double t = 0.0;
+  for (int k = lane >> 3; k < gp; k += 4) t += fpart[((long long)w * gp + k) * CP + q];
+  t += __shfl_xor_sync(0xffffffffu, t, 8);
+  t += __shfl_xor_sync(0xffffffffu, t, 16);
+  const int id = cid[gc * CP + q];
+  if (lane < CP && id >= 0) fbar[(long long)n * B + id] = t;
+}
+
+size_t obj_bytes(const mpc_ctx* c, int B, int steps, int ckpt) {
+  const size_t nch = (B + CP - 1) / CP, vec = 16 * nch * (size_t)c->g.ntot * CP;
+  const size_t nseg = (steps + ckpt - 1) / ckpt;
+  return vec * (nseg + 13 * (size_t)ckpt + kAdjSlots + 6) + 32 * (size_t)steps * B +
+         8 * nch * CP * (size_t)ckpt * c->num_sms;
+}
+
+}  // namespace
+
+// The batched objective runs here: faster than the stage GEMM, one launch.
+bool mpc_flowb_objective_wanted(mpc_ctx* c, int B) {
+  if (!mpc_flowb_wanted(c, B)) return false;
+  const int nch = (B + CP - 1) / CP;
+  return nch <= kMaxChunks * pick_groups(c->flowb, nch);
+}
+
+size_t mpc_flowb_objective_bytes(const mpc_ctx* c, int B, int steps, int ckpt) {
+  return obj_bytes(c, B, steps, ckpt);
+}
+
+// ckpt_every <= 0: the longest interval whose buffers fit in 85 % of the free
+// device memory.
+int mpc_flowb_auto_ckpt(mpc_ctx* c, int B, int steps, int* ckpt) {
+  mpc_flowb_state* f = c->flowb;
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  const double own = 16.0 * (f->ockp_n + f->oseg_n + f->V_n + f->xst_n + f->olam_n);
+  const double budget = 0.85 * ((double)free_b + own);
+  int k = steps;
+  while (k > 1 && (double)obj_bytes(c, B, steps, k) > budget) k = (k + 1) / 2;
+  if ((double)obj_bytes(c, B, steps, k) > budget)
+    return mpc_fail(MPC_ERR_NOMEM, "the batched objective needs %.3g GB, %.3g GB free",
+                    obj_bytes(c, B, steps, k) / 1e9, free_b / 1e9);
+  *ckpt = k;
+  return MPC_OK;
+}
+
+namespace {
+
+FbArgs obj_args(mpc_ctx* c) {
+  mpc_flowb_state* f = c->flowb;
+  FbArgs a{};
+  a.cid = f->oint;
+  a.csteps = f->oint + (size_t)f->onch * CP;
+  a.nsteps = a.csteps + f->onch;
+  a.in = f->oio;
+  a.out = f->oio + (size_t)f->oB * c->g.ntot;
+  a.Ftab = f->oF;
+  a.ldf = f->oB;
+  a.dt = f->odt;
+  a.pop_index = -1;
+  a.hist_ld = f->osteps;
+  a.norm_hist = f->onorm;
+  a.seg_v = f->oseg;
+  a.cvec = (long long)f->onch * c->g.ntot * CP;
+  return a;
+}
+
+// Steps [n0, n0 + len) of all pulses run: chunk and pulse step counts.
+int obj_steps(mpc_ctx* c, int len) {
+  mpc_flowb_state* f = c->flowb;
+  std::vector<int> v((size_t)f->onch + f->oB, len);
+  CK(cudaMemcpyAsync(f->oint + (size_t)f->onch * CP, v.data(), sizeof(int) * v.size(),
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));   // v is pageable and goes away
+  return MPC_OK;
+}
+
+int obj_status(mpc_ctx* c, const char* where) {
+  unsigned st = 0;
+  CK(cudaMemcpyAsync(&st, c->d_status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (!st) return MPC_OK;
+  CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+  return mpc_fail(MPC_ERR_DEVICE, "kernel status 0x%x during the %s", st, where);
+}
+
+}  // namespace
+
+// Forward pass of the batched objective: fields F host [steps][B], start
+// states ct0 host [B][n], final states into xN host [B][n].
+int mpc_flowb_objective(mpc_ctx* c, int B, const double* F, double dt, int steps, int ckpt,
+                        const double* ct0, double2* xN) {
+  mpc_flowb_state* f = c->flowb;
+  const size_t n = c->g.ntot;
+  const int nch = (B + CP - 1) / CP, nseg = (steps + ckpt - 1) / ckpt;
+  const size_t vec = (size_t)nch * n * CP;
+  int rc;
+  std::vector<int> cid((size_t)nch * CP, -1);
+  for (int i = 0; i < B; ++i) cid[i] = i;
+  f->oB = B;
+  f->osteps = steps;
+  f->ockpt = ckpt;
+  f->onch = nch;
+  f->ong = pick_groups(f, nch);
+  f->odt = dt;
+  f->okept = false;
+  if ((rc = grow(&f->oint, &f->oint_n, (size_t)nch * (CP + 1) + B)) ||
+      (rc = grow(&f->oio, &f->oio_n, 2 * B * n)) ||
+      (rc = grow(&f->oF, &f->oF_n, (size_t)steps * B)) ||
+      (rc = grow(&f->onorm, &f->onorm_n, (size_t)steps * B)) ||
+      (rc = grow(&f->ockp, &f->ockp_n, vec * nseg)) ||
+      (rc = grow(&f->oseg, &f->oseg_n, vec * 13 * std::min(ckpt, steps))) ||
+      (rc = grow(&f->olam, &f->olam_n, 2 * vec)) || (rc = grow(&f->ofs, &f->ofs_n, vec)) ||
+      (rc = grow(&f->ofp, &f->ofp_n,
+                 (size_t)std::min(ckpt, steps) * nch * f->grp[f->ong].gp * CP)) ||
+      (rc = grow(&f->ofb, &f->ofb_n, (size_t)steps * B)))
+    return rc;
+  CK(cudaMemcpyAsync(f->oio, ct0, sizeof(double2) * B * n, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->oF, F, sizeof(double) * (size_t)steps * B, cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(f->oint, cid.data(), sizeof(int) * cid.size(), cudaMemcpyHostToDevice,
+                     c->stream));
+  if ((rc = obj_steps(c, steps))) return rc;
+  FbArgs a = obj_args(c);
+  a.ckpt = f->ockp;
+  a.ckpt_every = ckpt;
+  a.seg_from = (nseg - 1) * ckpt;
+  if ((rc = launch(c, a, f->ong, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
+  CK(cudaMemcpyAsync(xN, a.out, sizeof(double2) * B * n, cudaMemcpyDeviceToHost, c->stream));
+  f->okept = true;
+  return obj_status(c, "batched forward pass");
+}
+
+// Its reverse pass: dJ/dF into fb host [steps][B].
+int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb) {
+  mpc_flowb_state* f = c->flowb;
+  const size_t n = c->g.ntot;
+  const int B = f->oB, nch = f->onch, steps = f->osteps, ckpt = f->ockpt;
+  const int nseg = (steps + ckpt - 1) / ckpt;
+  const size_t vec = (size_t)nch * n * CP;
+  int rc;
+  k_fb_seed<<<nch * CP, 256, 0, c->stream>>>(f->oint, f->oio + (size_t)B * n, c->d_eps, f->olam,
+                                             target, c->yield_thr, (int)n);
+  CK(cudaGetLastError());
+  ++c->launches;
+  int lens = -1;   // the step counts on the device
+  for (int seg = nseg - 1; seg >= 0; --seg) {
+    const int n0 = seg * ckpt, len = std::min(ckpt, steps - n0);
+    if (!(f->okept && seg == nseg - 1)) {
+      // recompute the segment's vectors, from the checkpoint and its norm
+      if (lens != len && (rc = obj_steps(c, lens = len))) return rc;
+      FbArgs a = obj_args(c);
+      a.start = f->ockp + vec * seg;
+      a.start_nrm = n0 > 0 ? f->onorm + (n0 - 1) : nullptr;
+      a.Ftab = f->oF + (size_t)n0 * B;
+      a.norm_hist = f->onorm + n0;   // the same norms again
+      a.out = f->oio;                // (the start states are not needed any more)
+      if ((rc = launch(c, a, f->ong, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
+    }
+    FbArgs a = obj_args(c);
+    a.Ftab = f->oF + (size_t)n0 * B;
+    a.norms = f->onorm + n0;
+    a.len = len;
+    a.lam = f->olam;
+    a.xb = f->olam + vec;
+    a.fs = f->ofs;
+    a.fpart = f->ofp;
+    if ((rc = launch(c, a, f->ong, nch, kAdjSlots, (const void*)&k_flow_batch<2>))) return rc;
+    k_fb_fbar<<<(len * nch * 32 + 127) / 128, 128, 0, c->stream>>>(
+        f->ofp, f->oint, len, nch, f->grp[f->ong].gp, f->ofb + (size_t)n0 * B, B);
+    CK(cudaGetLastError());
+    ++c->launches;
+  }
+  f->okept = f->okept && nseg == 1;   // the recomputes overwrote the last segment
+  CK(cudaMemcpyAsync(fb, f->ofb, sizeof(double) * (size_t)steps * B, cudaMemcpyDeviceToHost,
+                     c->stream));
+  return obj_status(c, "batched adjoint pass");
+}
 
 // Whether B pulses run faster here than on the stage GEMM.
 bool mpc_flowb_wanted(mpc_ctx* c, int B) {
@@ -271,50 +562,23 @@ int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
   CK(cudaMemcpyAsync(f->pulse, pulses, sizeof(mpc_pulse) * B, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(f->t0, t0, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
   FbArgs a{};
-  a.D = c->d_D;
-  a.eps = c->d_eps;
-  a.slots = kFixSlots;
-  a.status = c->d_status;
   a.in = in;
   a.out = out;
   a.pulse = f->pulse;
   a.t0 = f->t0;
   a.nsteps = f->ints + (ns - cid);
   a.dt = dt;
-  a.gauge = (c->gauge == 'l') ? 0 : 1;
   a.pop_index = pop_index;
   a.hist_ld = ld;
   a.pop_hist = pop_out ? f->hist : nullptr;
   a.norm_hist = norm_out ? f->hist + (pop_out ? hist : 0) : nullptr;
-  a.g = c->g;
   // launches of at most kMaxChunks chunks per column group
   for (int k0 = 0; k0 < nch_all;) {
     const int ng = pick_groups(f, nch_all - k0);
-    const Group& grp = f->grp[ng];
     const int nch = std::min(nch_all - k0, kMaxChunks * ng);
-    const size_t vn = (size_t)nch * kFixSlots * n * CP, pn = (size_t)nch * 2 * grp.gp * 2 * CP;
-    if ((rc = grow(&f->V, &f->V_n, vn)) || (rc = grow(&f->part, &f->part_n, pn)) ||
-        (rc = grow(&f->ctr, &f->ctr_n, (size_t)nch)) ||
-        (rc = grow(&f->xst, &f->xst_n, (size_t)nch * n * CP)))
-      return rc;
-    CK(cudaMemsetAsync(f->V, 0xff, sizeof(double2) * vn, c->stream));
-    CK(cudaMemsetAsync(f->part, 0xff, sizeof(double) * pn, c->stream));
-    CK(cudaMemsetAsync(f->ctr, 0, sizeof(unsigned long long) * nch, c->stream));
-    a.cta = grp.ctas;
-    a.gp = grp.gp;
-    a.ng = ng;
-    a.nch = nch;
     a.cid = f->ints + (size_t)k0 * CP;
     a.csteps = f->ints + (cst - cid) + k0;
-    a.V = f->V;
-    a.part = f->part;
-    a.ctr = f->ctr;
-    a.xst = f->xst;
-    a.bc = mpc_barrier_cfg(c);
-    void* args[] = {&a};
-    ProfScope ps(c, MPC_KERNEL_BATCH_STAGE);
-    CK(cudaLaunchCooperativeKernel((const void*)&k_flow_batch<0>, dim3(ng * grp.gp),
-                                   dim3(FTHREADS), args, flowb_smem(), c->stream));
+    if ((rc = launch(c, a, ng, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
     k0 += nch;
   }
   std::vector<double> h(pop_out || norm_out ? (pop_out ? hist : 0) + (norm_out ? hist : 0) : 0);

@@ -79,6 +79,21 @@ struct FbArgs {
   long long hist_ld;
   double* pop_hist;       // [id][hist_ld]
   double* norm_hist;      // [id][hist_ld]
+  // the objective gradient (null when unused).  Chunk vectors [nch][ntot][CP]
+  // lie cvec apart, the same vector of all chunks:
+  const double2* start;   // the first step's state, instead of `in`, ...
+  const double* start_nrm;  // ... and its norm by pulse id, hist_ld apart (null: 1)
+  double2* ckpt;          // slot k: x after k * ckpt_every steps, not yet renormalised
+  int ckpt_every;
+  double2* seg_v;         // step n >= seg_from: slot (n - seg_from) * 13 + m holds v_m, + 12 x_n
+  int seg_from;
+  long long cvec;
+  int len;                // mode 2: steps swept, the last first
+  const double* norms;    // mode 2: [id][hist_ld] norm of step n
+  double2* lam;           // mode 2: dJ/dx in and out
+  double2* xb;            // mode 2: the sum over m of G_m vbar_m
+  double* fs;             // mode 2: [nch][ntot][CP] dJ/dF of the step so far
+  double* fpart;          // mode 2: [len][nch][gp][CP]
   BarrierCfg bc;
   Geometry g;
 };
@@ -287,12 +302,15 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
   auto slot = [&](int c, int s) {
     return a.V + u.cpitch * (c * a.ng + u.grp) + u.spitch * s + (long long)u.row0 * CP;
   };
+  auto chunk = [&](int c) { return ((long long)(c * a.ng + u.grp) * a.g.ntot + u.row0) * CP; };
   // the start states, as given
   for (int c = 0; c < u.nc; ++c)
     for (int e = tid; e < ne; e += FT) {
       const int id = ctl.id[c][q];
-      publish(slot(c, fix_x(-1)) + e, id >= 0 ? a.in[(long long)id * a.g.ntot + u.row0 + (e >> 3)]
-                                              : make_double2(0.0, 0.0));
+      double2 x = make_double2(0.0, 0.0);
+      if (id >= 0)
+        x = a.start ? a.start[chunk(c) + e] : a.in[(long long)id * a.g.ntot + u.row0 + (e >> 3)];
+      publish(slot(c, fix_x(-1)) + e, x);
     }
   // items: per step, per product, the chunks with steps left (the longest first)
   int it = 0, act = u.nc;
@@ -335,7 +353,10 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
         // this thread's own elements of x and of the product's input
         double2 xo[NE], vo[NE];
         const double2* own = slot(c, in_slot);
-        double2* xs = a.xst + ((long long)(c * a.ng + u.grp) * a.g.ntot + u.row0) * CP;
+        double2* xs = a.xst + chunk(c);
+        double2* keep = a.seg_v && step >= a.seg_from
+                            ? a.seg_v + a.cvec * (13LL * (step - a.seg_from)) + chunk(c)
+                            : nullptr;
 #pragma unroll
         for (int i = 0; i < NE; ++i) {
           const int e = tid + i * FT;
@@ -357,8 +378,11 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
           const int row = u.row0 + (e >> 3);
           double2 W = fb_sum<MT>(rb, e), x = xo[i], v = vo[i];
           if (p == 0) {
+            if (a.ckpt && step % a.ckpt_every == 0)
+              a.ckpt[a.cvec * (step / a.ckpt_every) + chunk(c) + e] = v;
             x = fix_begin(a, ctl, c, q, row, step, v);
             xs[e] = x;
+            if (keep) keep[12 * a.cvec + e] = x;
             v = make_double2(sc * x.x, sc * x.y);   // v_12 = G_12 x
             W = quot2(W, ctl.nrm[c][q]);
             W.x *= sc;
@@ -367,6 +391,7 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
           const double2 m = fb_m(a.gauge, a.eps[row], F, v, W);
           const double2 o = make_double2(fma(h, m.x, gm * x.x), fma(h, m.y, gm * x.y));
           publish(dst + e, o);
+          if (keep && !last) keep[(11 - p) * a.cvec + e] = o;
           nsq += fma(o.x, o.x, o.y * o.y);
         }
         if (last) {
@@ -392,6 +417,37 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
   }
 }
 
+// Waits, as a warp, until *ctr reaches `target`; false after limit_ns.
+__device__ __forceinline__ bool fb_count(const unsigned long long* ctr, unsigned long long target,
+                                         int lane, unsigned long long limit_ns) {
+  bool ok = true;
+  if (lane == 0) {
+    unsigned long long v = 0, t0 = 0;
+    for (unsigned i = 0;; ++i) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ctr) : "memory");
+      if (v >= target) break;
+      if ((i & 1023u) == 1023u) {
+        const unsigned long long t = globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > limit_ns) {
+          ok = false;
+          break;
+        }
+      }
+    }
+  }
+  return __shfl_sync(0xffffffffu, ok, 0);
+}
+__device__ __forceinline__ void fb_arrive(unsigned long long* ctr) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(1ull) : "memory");
+}
+// Waits for the compute warps' `events`-th (step, chunk) pair.
+__device__ __forceinline__ bool fb_progress(FbCtl& ctl, int events) {
+  bool ok = true;
+  while (ok && ctl.progress < events) ok = ctl.mexit == 0 || ctl.progress >= events;
+  return __all_sync(0xffffffffu, ok);
+}
+
 // Per chunk and step: the norms from all CTAs' partials, the pulses' times and
 // next fields, the presets.  One warp; lane = (quarter of the CTAs, pulse).
 __device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, int lane) {
@@ -404,7 +460,10 @@ __device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, in
   };
   for (int c = 0; c < u.nc; ++c) {
     if (lane < CP) {
-      ctl.nrm[c][q] = make_double2(1.0, 1.0);
+      const double n0 = a.start_nrm && ctl.id[c][q] >= 0
+                            ? a.start_nrm[(long long)ctl.id[c][q] * a.hist_ld]
+                            : 1.0;
+      ctl.nrm[c][q] = make_double2(n0, 1.0 / n0);
       ctl.t[c][q] = ctl.id[c][q] >= 0 && a.t0 ? a.t0[ctl.id[c][q]] : 0.0;
       ctl.F[c][q] = field(c, 0);
     }
@@ -418,29 +477,11 @@ __device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, in
     for (int c = 0; c < u.nc && ctl.nst[c] > n; ++c) {
       any = true;
       ++events;
-      bool ok = true;
-      while (ok && ctl.progress < events) ok = ctl.mexit == 0;
-      ok = __all_sync(0xffffffffu, ok);
+      bool ok = fb_progress(ctl, events);
       if (!ok) return;
       const int gc = c * a.ng + u.grp;
-      if (n > 0) {   // everyone's presets of event n - 1 are made
-        if (lane == 0) {
-          unsigned long long v = 0, t0 = 0;
-          for (unsigned i = 0;; ++i) {
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a.ctr + gc) : "memory");
-            if (v >= (unsigned long long)n * a.gp + a.bc.skew) break;
-            if ((i & 1023u) == 1023u) {
-              const unsigned long long t = globaltimer_ns();
-              if (t0 == 0) t0 = t;
-              if (t - t0 > a.bc.wait_ns) {
-                ok = false;
-                break;
-              }
-            }
-          }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-      }
+      if (n > 0)   // everyone's presets of event n - 1 are made
+        ok = fb_count(a.ctr + gc, (unsigned long long)n * a.gp + a.bc.skew, lane, a.bc.wait_ns);
       double sum = 0.0;
       const double* pp = a.part + ((long long)gc * 2 + (n & 1)) * a.gp * (2 * CP);
       for (int b0 = lane >> 3; ok && b0 < a.gp; b0 += 32) {
@@ -503,12 +544,157 @@ __device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, in
         for (int e = lane; e < ne; e += 32) st_relaxed2(d + e, empty2());
       }
       __syncwarp();
-      if (lane == 0)
-        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(a.ctr + gc), "l"(1ull)
-                     : "memory");
+      if (lane == 0) fb_arrive(a.ctr + gc);
     }
     if (!any) return;
   }
+}
+
+// ---------------------------------------------------------------------------
+// the objective gradient's sweep (see k_flow_adjoint for the transposed
+// products): slots 3 x 12, ring m % 3 of the m-th swept step, vbar_p
+// ---------------------------------------------------------------------------
+constexpr int kAdjSlots = 36;
+__device__ __forceinline__ int adj_v(int m, int p) { return (m % 3) * 12 + p; }
+
+template <int MT, int KT>
+__device__ void fb_adj_main(const FbArgs& a, FbCtl& ctl, const FbView& u, double2* red,
+                            double (*red8)[CP], int tid) {
+  constexpr int NE = (MT * 64 + FT - 1) / FT;
+  const int warp = tid >> 5, lane = tid & 31, q = tid & 7;
+  FbTile<MT, KT> tile;
+  tile.init(a, u, warp, lane);
+  const double h = a.dt;
+  const int ne = u.nrows * CP;
+  auto slot = [&](int c, int s) {
+    return a.V + u.cpitch * (c * a.ng + u.grp) + u.spitch * s + (long long)u.row0 * CP;
+  };
+  auto chunk = [&](int c) { return ((long long)(c * a.ng + u.grp) * a.g.ntot + u.row0) * CP; };
+  // zbar = lambda / ||z_n|| of the step with local index n
+  auto zbar = [&](int c, int n, double2 l) {
+    const int id = ctl.id[c][q];
+    const double nz = id >= 0 ? a.norms[(long long)id * a.hist_ld + n] : 1.0;
+    return quot2(l, make_double2(nz, 1.0 / nz));
+  };
+  for (int c = 0; c < u.nc; ++c)
+    for (int e = tid; e < ne; e += FT)
+      publish(slot(c, adj_v(0, 0)) + e, zbar(c, a.len - 1, a.lam[chunk(c) + e]));
+  int it = 0;
+  bool primed = false;
+  for (int m = 0; m < a.len; ++m) {
+    const int n = a.len - 1 - m;   // the step, counted from the segment's start
+#pragma unroll 1
+    for (int p = 0; p < kFlowProducts; ++p) {
+      const bool last = p == kFlowProducts - 1;
+      const double gm = f_G[p], sc = last ? f_G[12] : 1.0;
+#pragma unroll 1
+      for (int c = 0; c < u.nc; ++c, ++it) {
+        if (p == 0 && !fb_await(ctl, c, m - 1)) ctl.mdead[it & 1] = 1;
+        const double2* src = fb_slot(a, u, c, adj_v(m, p));
+        if (!primed) tile.prefetch(src);
+        double acc[MT][4];
+        tile.run(src, acc, &ctl.mdead[it & 1], a.status, a.bc.wait_ns);
+        // (a step's first product waits for the helper's word, chunk by chunk)
+        primed = u.nc > 1 && (c + 1 < u.nc ? p > 0 : !last);
+        if (primed)
+          tile.prefetch(c + 1 < u.nc ? fb_slot(a, u, c + 1, adj_v(m, p))
+                                     : fb_slot(a, u, 0, adj_v(m, p + 1)));
+        double2* rb = red + (it & 1) * (FW * MT * 64);
+        tile.put(acc, rb, warp, lane);
+        double2 vo[NE], vk[NE], xo[NE];
+        double fo[NE];
+        const double2* own = slot(c, adj_v(m, p));
+        const double2* kept = a.seg_v + a.cvec * (13LL * n + p + 1) + chunk(c);
+        double2* xs = a.xb + chunk(c);
+        double* fv = a.fs + chunk(c);
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e < ne) {
+            vo[i] = __ldcg(own + e);
+            vk[i] = kept[e];
+            if (p > 0) {
+              xo[i] = xs[e];
+              fo[i] = fv[e];
+            }
+          }
+        }
+        named_bar_sync(kBarMain, FT);
+        if (ctl.mdead[it & 1]) return;
+        const double F = ctl.id[c][q] >= 0 ? a.Ftab[(long long)n * a.ldf + ctl.id[c][q]] : 0.0;
+        double fsum = 0.0;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e >= ne) continue;
+          const double2 W = fb_sum<MT>(rb, e), vb = vo[i];
+          const double2 m1 = a.gauge == 0 ? make_double2(W.y, -W.x) : W;
+          const double2 mv = fb_m(a.gauge, a.eps[u.row0 + (e >> 3)], F, vb, W);
+          const double2 o = make_double2(-h * mv.x, -h * mv.y);   // vbar_{p+1}
+          double2 x = p > 0 ? xo[i] : make_double2(0.0, 0.0);
+          x.x = fma(gm, vb.x, x.x);
+          x.y = fma(gm, vb.y, x.y);
+          double f = p > 0 ? fo[i] : 0.0;
+          f -= sc * fma(m1.x, vk[i].x, m1.y * vk[i].y);   // v_12 = G_12 x
+          if (!last) {
+            publish(slot(c, adj_v(m, p + 1)) + e, o);
+            xs[e] = x;
+            fv[e] = f;
+          } else {
+            const double2 l = make_double2(fma(f_G[12], o.x, x.x), fma(f_G[12], o.y, x.y));
+            fsum += f * h;
+            if (m + 1 < a.len)
+              publish(slot(c, adj_v(m + 1, 0)) + e, zbar(c, n - 1, l));
+            else
+              a.lam[chunk(c) + e] = l;
+          }
+        }
+        if (last) {
+          fsum += __shfl_xor_sync(0xffffffffu, fsum, 8);
+          fsum += __shfl_xor_sync(0xffffffffu, fsum, 16);
+          if (lane < CP) red8[warp][lane] = fsum;
+          named_bar_sync(kBarMain, FT);
+          if (tid < CP) {
+            double t = red8[0][tid];
+#pragma unroll
+            for (int k = 1; k < FW; ++k) t += red8[k][tid];
+            a.fpart[(((long long)n * a.nch + c * a.ng + u.grp) * a.gp + u.idx) * CP + tid] = t;
+          }
+          if (tid == 0) ctl.progress = ctl.progress + 1;
+        }
+      }
+    }
+  }
+}
+
+// Once every CTA is past a chunk's m-th step its ring is preset, for the step
+// m + 3; the arrival of the next step publishes that.
+__device__ void fb_adj_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, int lane) {
+  int events = 0;
+  for (int m = 0; m < a.len; ++m)
+    for (int c = 0; c < u.nc; ++c) {
+      if (!fb_progress(ctl, ++events)) return;
+      const int gc = c * a.ng + u.grp;
+      __syncwarp();
+      if (lane == 0) fb_arrive(a.ctr + gc);
+      if (!fb_count(a.ctr + gc, (unsigned long long)(m + 1) * a.gp + a.bc.skew, lane,
+                    a.bc.wait_ns)) {
+        if (lane == 0) {
+          atomicOr(a.status, ST_WAIT_TIMEOUT);
+          ctl.hdead = 1;
+        }
+        return;
+      }
+      double2* base = a.V + u.cpitch * gc + (long long)u.row0 * CP;
+      const int ne = u.nrows * CP;
+      for (int p = 0; p < 12; ++p) {
+        double2* d = base + u.spitch * adj_v(m, p);
+        for (int e = lane; e < ne; e += 32) st_relaxed2(d + e, empty2());
+      }
+      __syncwarp();
+      __threadfence_block();
+      if (lane == 0) ctl.step[c] = m + 1;
+    }
 }
 
 template <int MODE>
@@ -536,7 +722,7 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constan
     ctl.ns[c][q] = id >= 0 && a.nsteps ? a.nsteps[id] : 0;
     if (q == 0) {
       ctl.nst[c] = a.csteps[c * a.ng + me.grp];
-      ctl.step[c] = -1;
+      ctl.step[c] = MODE == 2 ? 0 : -1;
     }
   }
   if (tid == 0) {
@@ -550,12 +736,20 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constan
   X(8, 2, 19) X(9, 3, 19) X(10, 2, 25) X(11, 3, 25)
   if (warp >= FW) {
     regs_dec<40>();
-    if (warp == FW) fb_fixed_helper(a, ctl, u, lane);
+    if (warp == FW) {
+      if constexpr (MODE == 2)
+        fb_adj_helper(a, ctl, u, lane);
+      else
+        fb_fixed_helper(a, ctl, u, lane);
+    }
     return;
   }
   regs_inc<232>();
 #define FB_RUN(I, MT, KT) \
-  case I: fb_fixed_main<MT, KT>(a, ctl, u, red, red8, tid); break;
+  case I: \
+    if constexpr (MODE == 2) fb_adj_main<MT, KT>(a, ctl, u, red, red8, tid); \
+    else fb_fixed_main<MT, KT>(a, ctl, u, red, red8, tid); \
+    break;
   switch (me.cfg) { FB_CONFIGS(FB_RUN) }
 #undef FB_RUN
   if (tid == 0) ctl.mexit = 1;

@@ -11,3 +11,11 @@ void mpc_flowb_free(mpc_ctx* c);
 int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
                       const int* steps, int pop_index, double* ct, double* pop_out,
                       double* norm_out, int max_steps);
+
+// The batched objective on the same kernels (see flow_batch.cu).
+bool mpc_flowb_objective_wanted(mpc_ctx* c, int B);
+size_t mpc_flowb_objective_bytes(const mpc_ctx* c, int B, int steps, int ckpt);
+int mpc_flowb_auto_ckpt(mpc_ctx* c, int B, int steps, int* ckpt);
+int mpc_flowb_objective(mpc_ctx* c, int B, const double* F, double dt, int steps, int ckpt,
+                        const double* ct0, double2* xN);
+int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb);

@@ -53,3 +53,29 @@ def test_fixed_steps_match_single_pulse(n, B, gauge):
             assert np.max(np.abs(pop[b, :k + 1] - p1)) < 6e-13 * k, b
             assert np.max(np.abs(nrm[b, :k] - n1)) < 6e-13 * k, b
             assert np.all(np.isnan(nrm[b, k:])) and np.all(np.isnan(pop[b, k + 1:]))
+
+
+@pytest.mark.parametrize("gauge", ["l", "v"])
+@pytest.mark.parametrize("B", [1, 9, 20])
+@pytest.mark.parametrize("n", SYSTEMS, ids=lambda n: f"{len(n)}x{max(n)}")
+def test_gradient_matches_single_pulse(n, B, gauge):
+    """Gradients relative to the largest component (both factors of each
+    Re<M1 vbar, v> carry the bound above: 1e-11 over 5 steps); segments of one
+    step, shorter than the window, and one for all; a second reverse pass."""
+    s, pulses, X = _case(n, gauge, B)
+    U = np.random.default_rng(3).standard_normal((B, 6)) * 1e-3
+    T = np.full(B, 2.0)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        first = None
+        for steps, ckpt in ((1, 64), (5, 2), (5, 64), (5, 1)):
+            J, G, Fb = ctx.batch_objective_gradient(pulses, U, T, 0.1, 0.1, steps, X, 0, ckpt)
+            G2, Fb2 = ctx.batch_objective_backward()
+            assert np.array_equal(G, G2) and np.array_equal(Fb, Fb2)
+            if steps == 5:
+                first = first or (J, G, Fb)
+                assert all(np.array_equal(x, y) for x, y in zip(first, (J, G, Fb)))
+            for b in range(0, B, 4):
+                j, g, f = ctx.objective_gradient(pulses[b], U[b], 2.0, 0.1, 0.1, steps, X[b], 0)
+                assert abs(J[b] - j) < 4e-12
+                assert np.max(np.abs(Fb[b] - f)) <= 1e-11 * max(np.max(np.abs(f)), 1e-3)
+                assert np.max(np.abs(G[b] - g)) <= 1e-11 * max(np.max(np.abs(g)), 1e-3)
