@@ -1148,6 +1148,10 @@ int mpc_batch_propagate(mpc_ctx* c, int B, const mpc_pulse* pulses, const double
     return mpc_fail(MPC_ERR_UNSTABLE,
                     "dt_max*max|E| = %.4g exceeds the RKF78 imaginary-axis stability bound %.4g",
                     dt_max * c->eps_max, kRk78ImagStability);
+  CK(cudaSetDevice(c->device));
+  if (mpc_flowb_wanted(c, B))
+    return mpc_flowb_propagate(c, B, pulses, t0, t_end, h0, dt_max, rtol, atol, max_attempts, ct,
+                               accepted, rejected, t_final);
   FixedStep fx{};
   return batch_run(c, B, pulses, t0, t_end, h0, dt_max, rtol, atol, max_attempts, ct, accepted,
                    rejected, t_final, fx, nullptr);

@@ -18,6 +18,10 @@ using namespace mpc;
 namespace {
 
 constexpr int kMaxGroups = 4;
+const void* const kKernels[] = {reinterpret_cast<const void*>(&k_flow_batch<0>),
+                                reinterpret_cast<const void*>(&k_flow_batch<1>),
+                                reinterpret_cast<const void*>(&k_flow_batch<2>)};
+const int kSlots[] = {kFixSlots, kAdaptSlots, kAdjSlots};
 
 int window_len(const Geometry& g, int L) {
   return (L > 0 ? g.state_off[L] - g.state_off[L - 1] : 0) +
@@ -113,6 +117,7 @@ struct Group {
   bool ok = false;
   int gp = 0;       // CTAs per group
   int cost = 0;
+  int mt = 0, rows = 0;   // of its largest CTA
   FbCta* ctas = nullptr;
 };
 
@@ -131,6 +136,7 @@ int grow(T** p, size_t* cap, size_t n) {
 
 struct mpc_flowb_state {
   bool tried = false, ok = false;
+  size_t optin = 0;          // shared memory a CTA may have
   Group grp[kMaxGroups + 1];
   // work space, kept between calls and grown on demand
   double2* V = nullptr;
@@ -141,6 +147,8 @@ struct mpc_flowb_state {
   size_t ctr_n = 0;
   double2* xst = nullptr;
   size_t xst_n = 0;
+  double2* kst = nullptr;    // adaptive steps: slopes and x_new
+  size_t kst_n = 0;
   double2* io = nullptr;     // start and final states by pulse id
   size_t io_n = 0;
   int* ints = nullptr;       // chunk ids, chunk steps, pulse steps
@@ -188,7 +196,19 @@ bool mpc_flowb_setup(mpc_ctx* c) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   if (!coop) return false;
-  if (cudaMemcpyToSymbol(f_G, rkf78::G, sizeof rkf78::G) != cudaSuccess) {
+  f->optin = optin;
+  double A[13][13], B8[13], E[13], Cn[13];
+  for (int i = 0; i < 13; ++i) {
+    for (int j = 0; j < 13; ++j) A[i][j] = rkf78::A[i][j];
+    B8[i] = rkf78::B8[i];
+    E[i] = rkf78::B8[i] - rkf78::B7[i];
+    Cn[i] = rkf78::C[i];
+  }
+  if (cudaMemcpyToSymbol(f_G, rkf78::G, sizeof rkf78::G) != cudaSuccess ||
+      cudaMemcpyToSymbol(f_A, A, sizeof A) != cudaSuccess ||
+      cudaMemcpyToSymbol(f_B8, B8, sizeof B8) != cudaSuccess ||
+      cudaMemcpyToSymbol(f_E, E, sizeof E) != cudaSuccess ||
+      cudaMemcpyToSymbol(f_C, Cn, sizeof Cn) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -201,16 +221,17 @@ bool mpc_flowb_setup(mpc_ctx* c) {
       for (FbCta t : one) {
         t.grp = k;
         all.push_back(t);
+        g.mt = std::max(g.mt, kConfigs[t.cfg].mt);
+        g.rows = std::max(g.rows, t.nrows);
       }
     int per_sm = 0;
-    if (!mpc_allow_smem((const void*)&k_flow_batch<0>, optin) ||
-        !mpc_allow_smem((const void*)&k_flow_batch<2>, optin) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flow_batch<0>, FTHREADS,
-                                                      flowb_smem()) != cudaSuccess ||
-        per_sm < 1 ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flow_batch<2>, FTHREADS,
-                                                      flowb_smem()) != cudaSuccess ||
-        per_sm < 1 || cudaMalloc(&g.ctas, sizeof(FbCta) * all.size()) != cudaSuccess ||
+    bool fits = true;
+    for (int mode = 0; mode < 3 && fits; ++mode)
+      fits = mpc_allow_smem(kKernels[mode], optin) &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernels[mode], FTHREADS,
+                                                           flowb_smem(mode, g.mt)) == cudaSuccess &&
+             per_sm >= 1;
+    if (!fits || cudaMalloc(&g.ctas, sizeof(FbCta) * all.size()) != cudaSuccess ||
         cudaMemcpy(g.ctas, all.data(), sizeof(FbCta) * all.size(), cudaMemcpyHostToDevice) !=
             cudaSuccess) {
       cudaGetLastError();
@@ -230,6 +251,7 @@ void mpc_flowb_free(mpc_ctx* c) {
   cudaFree(f->part);
   cudaFree(f->ctr);
   cudaFree(f->xst);
+  cudaFree(f->kst);
   cudaFree(f->io);
   cudaFree(f->ints);
   cudaFree(f->pulse);
@@ -271,7 +293,8 @@ int pick_groups(const mpc_flowb_state* f, int nch) {
 namespace {
 
 // One launch of nch chunks on ng column groups, its work space preset.
-int launch(mpc_ctx* c, FbArgs& a, int ng, int nch, int slots, const void* kernel) {
+int launch(mpc_ctx* c, FbArgs& a, int ng, int nch, int mode, int slope_chunks = 0) {
+  const int slots = kSlots[mode];
   mpc_flowb_state* f = c->flowb;
   const Group& grp = f->grp[ng];
   const size_t n = c->g.ntot;
@@ -291,6 +314,7 @@ int launch(mpc_ctx* c, FbArgs& a, int ng, int nch, int slots, const void* kernel
   a.g = c->g;
   a.cta = grp.ctas;
   a.gp = grp.gp;
+  a.mt = grp.mt;
   a.ng = ng;
   a.nch = nch;
   a.V = f->V;
@@ -300,8 +324,8 @@ int launch(mpc_ctx* c, FbArgs& a, int ng, int nch, int slots, const void* kernel
   a.bc = mpc_barrier_cfg(c);
   void* args[] = {&a};
   ProfScope ps(c, MPC_KERNEL_BATCH_STAGE);
-  CK(cudaLaunchCooperativeKernel(kernel, dim3(ng * grp.gp), dim3(FTHREADS), args, flowb_smem(),
-                                 c->stream));
+  CK(cudaLaunchCooperativeKernel(kKernels[mode], dim3(ng * grp.gp), dim3(FTHREADS), args,
+                                 flowb_smem(mode, grp.mt, slope_chunks, grp.rows), c->stream));
   return MPC_OK;
 }
 
@@ -468,7 +492,7 @@ int mpc_flowb_objective(mpc_ctx* c, int B, const double* F, double dt, int steps
   a.ckpt = f->ockp;
   a.ckpt_every = ckpt;
   a.seg_from = (nseg - 1) * ckpt;
-  if ((rc = launch(c, a, f->ong, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
+  if ((rc = launch(c, a, f->ong, nch, 0))) return rc;
   CK(cudaMemcpyAsync(xN, a.out, sizeof(double2) * B * n, cudaMemcpyDeviceToHost, c->stream));
   f->okept = true;
   return obj_status(c, "batched forward pass");
@@ -498,7 +522,7 @@ int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb) {
       a.Ftab = f->oF + (size_t)n0 * B;
       a.norm_hist = f->onorm + n0;   // the same norms again
       a.out = f->oio;                // (the start states are not needed any more)
-      if ((rc = launch(c, a, f->ong, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
+      if ((rc = launch(c, a, f->ong, nch, 0))) return rc;
     }
     FbArgs a = obj_args(c);
     a.Ftab = f->oF + (size_t)n0 * B;
@@ -508,7 +532,7 @@ int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb) {
     a.xb = f->olam + vec;
     a.fs = f->ofs;
     a.fpart = f->ofp;
-    if ((rc = launch(c, a, f->ong, nch, kAdjSlots, (const void*)&k_flow_batch<2>))) return rc;
+    if ((rc = launch(c, a, f->ong, nch, 2))) return rc;
     k_fb_fbar<<<(len * nch * 32 + 127) / 128, 128, 0, c->stream>>>(
         f->ofp, f->oint, len, nch, f->grp[f->ong].gp, f->ofb + (size_t)n0 * B, B);
     CK(cudaGetLastError());
@@ -578,7 +602,7 @@ int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
     const int nch = std::min(nch_all - k0, kMaxChunks * ng);
     a.cid = f->ints + (size_t)k0 * CP;
     a.csteps = f->ints + (cst - cid) + k0;
-    if ((rc = launch(c, a, ng, nch, kFixSlots, (const void*)&k_flow_batch<0>))) return rc;
+    if ((rc = launch(c, a, ng, nch, 0))) return rc;
     k0 += nch;
   }
   std::vector<double> h(pop_out || norm_out ? (pop_out ? hist : 0) + (norm_out ? hist : 0) : 0);
@@ -603,5 +627,84 @@ int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
   }
   CK(cudaMemcpyAsync(ct, out, sizeof(double2) * (size_t)B * n, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  return MPC_OK;
+}
+
+// The adaptive propagation of B pulses (mpc_batch_propagate); ct host [B][n] in
+// and out, results by pulse (host).
+int mpc_flowb_propagate(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0,
+                        const double* t_end, double h0, double dt_max, double rtol, double atol,
+                        int max_attempts, double* ct, int* accepted, int* rejected,
+                        double* t_final) {
+  mpc_flowb_state* f = c->flowb;
+  const size_t n = c->g.ntot;
+  int rc;
+  // pulses by the time they have to run: a chunk goes on until its last is done
+  std::vector<int> order(B);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return t_end[x] - t0[x] > t_end[y] - t0[y]; });
+  const int nch_all = (B + CP - 1) / CP;
+  std::vector<int> ints((size_t)nch_all * (CP + 1) + 3 * (size_t)B, 0);
+  int* cid = ints.data();
+  std::fill(cid, cid + (size_t)nch_all * CP, -1);
+  std::copy(order.begin(), order.end(), cid);
+  const size_t res = (size_t)nch_all * (CP + 1);   // nacc, nrej, gave_up
+  if ((rc = grow(&f->ints, &f->ints_n, ints.size())) || (rc = grow(&f->pulse, &f->pulse_n, (size_t)B)) ||
+      (rc = grow(&f->t0, &f->t0_n, 3 * (size_t)B)) || (rc = grow(&f->io, &f->io_n, 2 * B * n)))
+    return rc;
+  CK(cudaMemcpyAsync(f->io, ct, sizeof(double2) * B * n, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->ints, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(f->pulse, pulses, sizeof(mpc_pulse) * B, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->t0, t0, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->t0 + B, t_end, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
+  FbArgs a{};
+  a.in = f->io;
+  a.out = f->io + B * n;
+  a.pulse = f->pulse;
+  a.t0 = f->t0;
+  a.t_end = f->t0 + B;
+  a.h0 = h0;
+  a.dt_max = dt_max;
+  a.rtol = rtol;
+  a.atol = atol;
+  a.max_attempts = max_attempts > 0 ? max_attempts : 1000000000;
+  a.nacc = f->ints + res;
+  a.nrej = a.nacc + B;
+  a.gave_up = a.nrej + B;
+  a.tf = f->t0 + 2 * (size_t)B;
+  for (int k0 = 0; k0 < nch_all;) {
+    const int ng = pick_groups(f, nch_all - k0);
+    const int nch = std::min(nch_all - k0, kMaxAdapt * ng), per = (nch + ng - 1) / ng;
+    const size_t vec = (size_t)nch * n * CP;
+    const Group& grp = f->grp[ng];
+    const bool shm = flowb_smem(1, grp.mt, per, grp.rows) + 1024 <= f->optin;
+    if ((rc = grow(&f->kst, &f->kst_n, vec * kNumStages))) return rc;
+    a.cid = f->ints + (size_t)k0 * CP;
+    a.csteps = f->ints + (size_t)nch_all * CP;   // unused: zeros
+    a.xnew = f->kst;
+    a.kst = shm ? nullptr : f->kst + vec;
+    a.cvec = (long long)vec;
+    if ((rc = launch(c, a, ng, nch, 1, shm ? per : 0))) return rc;
+    k0 += nch;
+  }
+  std::vector<double> tf(B);
+  CK(cudaMemcpyAsync(ints.data() + res, f->ints + res, sizeof(int) * 3 * (size_t)B,
+                     cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(tf.data(), a.tf, sizeof(double) * B, cudaMemcpyDeviceToHost, c->stream));
+  if ((rc = obj_status(c, "batched propagation"))) return rc;
+  CK(cudaMemcpyAsync(ct, a.out, sizeof(double2) * B * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  int gave_up = 0;
+  for (int b = 0; b < B; ++b) {
+    if (accepted) accepted[b] = ints[res + b];
+    if (rejected) rejected[b] = ints[res + B + b];
+    if (t_final) t_final[b] = tf[b];
+    gave_up += ints[res + 2 * (size_t)B + b];
+  }
+  if (gave_up)
+    return mpc_fail(MPC_ERR_DEVICE, "%d pulse(s) stopped after max_attempts step attempts",
+                    gave_up);
   return MPC_OK;
 }

@@ -62,6 +62,7 @@ struct FbArgs {
   const int* csteps;      // [nch] steps of the chunk's longest pulse (descending per group)
   double2* V;             // [nch][slots][ntot][CP] vectors in flight
   int slots;
+  int mt;                 // most 8-row tiles of a CTA
   double* part;           // [nch][2][gp][2 * CP] norm (and error) partials
   unsigned long long* ctr;  // [nch] helpers' arrivals
   unsigned* status;
@@ -94,6 +95,16 @@ struct FbArgs {
   double2* xb;            // mode 2: the sum over m of G_m vbar_m
   double* fs;             // mode 2: [nch][ntot][CP] dJ/dF of the step so far
   double* fpart;          // mode 2: [len][nch][gp][CP]
+  // adaptive steps
+  const double* t_end;    // by pulse id
+  double h0, dt_max, rtol, atol;
+  int max_attempts;
+  double2* kst;           // [12] slopes, cvec apart; null: in shared memory
+  double2* xnew;          // the attempt's x_new
+  int* nacc;              // results by pulse id
+  int* nrej;
+  double* tf;
+  int* gave_up;
   BarrierCfg bc;
   Geometry g;
 };
@@ -117,6 +128,21 @@ struct FbCtl {
   volatile int progress;         // (step, chunk) pairs the compute warps finished
   volatile int hdead, mexit;
   volatile int mdead[2];         // a wait ran out, by item parity
+};
+
+// What adaptive steps need besides.
+constexpr int kMaxAdapt = 16;       // chunks per column group and launch
+struct FbAdapt {
+  double F[kMaxAdapt][kNumStages][CP];   // the attempt's stage fields
+  double h[kMaxAdapt][CP];      // proposed next step
+  double hatt[kMaxAdapt][CP];   // step of the attempt
+  double t_end[kMaxAdapt][CP];
+  int acc[kMaxAdapt][CP];       // the last attempt was accepted
+  int ret[kMaxAdapt][CP];       // the pulse ended with it
+  int done[kMaxAdapt][CP];      // 1 at t_end, 2 gave up, 3 empty slot
+  int lastst[kMaxAdapt][CP];    // the attempt ends at t_end
+  int cnt[kMaxAdapt][3][CP];    // accepted, rejected, attempts
+  int alive[kMaxAdapt];         // the chunk has pulses left
 };
 
 struct FbView {
@@ -697,13 +723,338 @@ __device__ void fb_adj_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, int 
     }
 }
 
+// ---------------------------------------------------------------------------
+// adaptive steps: slots 2 x 13 stage inputs by attempt parity
+// ---------------------------------------------------------------------------
+constexpr int kAdaptSlots = 26;
+__device__ __forceinline__ int ada_y(int att, int s) { return (att & 1) * kNumStages + s; }
+
+static __constant__ double f_A[13][13];
+static __constant__ double f_B8[13];
+static __constant__ double f_E[13];   // b8 - b7
+static __constant__ double f_C[13];
+
+__device__ __forceinline__ double fb_nanmax(double m, double e) {
+  return (m != m) ? m : ((e != e) ? e : fmax(m, e));
+}
+
+template <int MT, int KT>
+__device__ void fb_adapt_main(const FbArgs& a, FbCtl& ctl, FbAdapt& ad, const FbView& u,
+                              double2* red, double2* kshm, double (*red8)[CP], double (*rede)[CP],
+                              int tid) {
+  constexpr int NE = (MT * 64 + FT - 1) / FT;
+  const int warp = tid >> 5, lane = tid & 31, q = tid & 7;
+  FbTile<MT, KT> tile;
+  tile.init(a, u, warp, lane);
+  const int ne = u.nrows * CP;
+  auto slot = [&](int c, int s) {
+    return a.V + u.cpitch * (c * a.ng + u.grp) + u.spitch * s + (long long)u.row0 * CP;
+  };
+  auto chunk = [&](int c) { return ((long long)(c * a.ng + u.grp) * a.g.ntot + u.row0) * CP; };
+  for (int c = 0; c < u.nc; ++c)
+    for (int e = tid; e < ne; e += FT) {
+      const int id = ctl.id[c][q];
+      a.xst[chunk(c) + e] = id >= 0 ? a.in[(long long)id * a.g.ntot + u.row0 + (e >> 3)]
+                                    : make_double2(0.0, 0.0);
+    }
+  unsigned live = u.nc >= 32 ? 0xffffffffu : (1u << u.nc) - 1u;
+  int it = 0;
+  bool primed = false;
+  for (int att = 0;; ++att) {
+    // ---- the attempt's start states out: x_new / ||x_new|| where the last
+    // attempt was accepted; finished pulses leave ----
+    for (int c = 0; c < u.nc; ++c) {
+      if (!(live >> c & 1u)) continue;
+      const bool ok = fb_await(ctl, c, att);
+      if (!ok) ctl.mdead[it & 1] = 1;
+      const int id = ctl.id[c][q];
+      for (int e = tid; e < ne && ok; e += FT) {
+        double2 x = a.xst[chunk(c) + e];
+        if (ad.acc[c][q]) {
+          x = quot2(a.xnew[chunk(c) + e], ctl.nrm[c][q]);
+          a.xst[chunk(c) + e] = x;
+        }
+        if (ad.ret[c][q]) a.out[(long long)id * a.g.ntot + u.row0 + (e >> 3)] = x;
+        if (ad.alive[c]) publish(slot(c, ada_y(att, 0)) + e, x);
+      }
+      if (ok && !ad.alive[c]) live &= ~(1u << c);
+    }
+    if (!live) return;
+#pragma unroll 1
+    for (int s = 0; s < kNumStages; ++s) {
+      const bool last = s == kNumStages - 1;
+#pragma unroll 1
+      for (unsigned todo = live; todo; todo &= todo - 1) {
+        const int c = __ffs(todo) - 1;
+        const unsigned after = todo & (todo - 1);
+        const double2* src = fb_slot(a, u, c, ada_y(att, s));
+        if (!primed) tile.prefetch(src);
+        double acc[MT][4];
+        tile.run(src, acc, &ctl.mdead[it & 1], a.status, a.bc.wait_ns);
+        primed = (live & (live - 1)) && (after || !last);
+        if (primed)
+          tile.prefetch(after ? fb_slot(a, u, __ffs(after) - 1, ada_y(att, s))
+                              : fb_slot(a, u, __ffs(live) - 1, ada_y(att, s + 1)));
+        double2* rb = red + (it & 1) * (FW * MT * 64);
+        tile.put(acc, rb, warp, lane);
+        double2 xo[NE], vo[NE];
+        const double2* own = slot(c, ada_y(att, s));
+        double2* ks = kshm ? kshm + c * (kNumStages - 1) * ne : a.kst + chunk(c);
+        const long long kp = kshm ? ne : a.cvec;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e < ne) {
+            vo[i] = __ldcg(own + e);
+            xo[i] = a.xst[chunk(c) + e];
+          }
+        }
+        named_bar_sync(kBarMain, FT);
+        if (ctl.mdead[it & 1]) return;
+        const double F = ad.F[c][s][q], hq = ad.hatt[c][q];
+        double nsq = 0.0, em = 0.0;
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+          const int e = tid + i * FT;
+          if (e >= ne) continue;
+          const double2 x = xo[i];
+          const double2 k = fb_m(a.gauge, a.eps[u.row0 + (e >> 3)], F, vo[i], fb_sum<MT>(rb, e));
+          if (!last) ks[s * kp + e] = k;
+          double2 o = x;
+          if (!last) {
+#pragma unroll
+            for (int j = 0; j < kNumStages - 1; ++j) {
+              const double cj = f_A[s + 1][j];
+              if (j > s || cj == 0.0) continue;
+              const double2 w = j == s ? k : ks[j * kp + e];
+              const double cf = hq * cj;
+              o.x = fma(cf, w.x, o.x);
+              o.y = fma(cf, w.y, o.y);
+            }
+            publish(slot(c, ada_y(att, s + 1)) + e, o);
+          } else {
+            double2 er = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int j = 0; j < kNumStages; ++j) {
+              const double bj = f_B8[j], ej = f_E[j];
+              if (bj == 0.0 && ej == 0.0) continue;
+              const double2 w = j == kNumStages - 1 ? k : ks[j * kp + e];
+              if (bj != 0.0) {
+                o.x = fma(hq * bj, w.x, o.x);
+                o.y = fma(hq * bj, w.y, o.y);
+              }
+              if (ej != 0.0) {
+                er.x = fma(hq * ej, w.x, er.x);
+                er.y = fma(hq * ej, w.y, er.y);
+              }
+            }
+            const double ax = sqrt(x.x * x.x + x.y * x.y), an = sqrt(o.x * o.x + o.y * o.y);
+            const double ae = sqrt(er.x * er.x + er.y * er.y);
+            em = fb_nanmax(em, ae / (a.atol + a.rtol * fmax(ax, an)));
+            a.xnew[chunk(c) + e] = o;
+            nsq += o.x * o.x + o.y * o.y;
+          }
+        }
+        if (last) {
+          nsq += __shfl_xor_sync(0xffffffffu, nsq, 8);
+          nsq += __shfl_xor_sync(0xffffffffu, nsq, 16);
+          em = fb_nanmax(em, __shfl_xor_sync(0xffffffffu, em, 8));
+          em = fb_nanmax(em, __shfl_xor_sync(0xffffffffu, em, 16));
+          if (lane < CP) {
+            red8[warp][lane] = nsq;
+            rede[warp][lane] = em;
+          }
+          named_bar_sync(kBarMain, FT);
+          if (tid < CP) {
+            double t = red8[0][tid], m = rede[0][tid];
+#pragma unroll
+            for (int k = 1; k < FW; ++k) {
+              t += red8[k][tid];
+              m = fb_nanmax(m, rede[k][tid]);
+            }
+            double* pp = a.part + (((long long)(c * a.ng + u.grp) * 2 + (att & 1)) * a.gp + u.idx) *
+                                      (2 * CP) + tid;
+            st_relaxed1(pp, canonical(t));
+            st_relaxed1(pp + CP, canonical(m));
+          }
+          __syncwarp();
+          if (tid == 0) ctl.progress = ctl.progress + 1;
+        }
+        ++it;
+      }
+    }
+  }
+}
+
+// Per chunk and attempt: norm and error over all CTAs, accept or reject, the
+// next step and its stage fields (the controller of the stage-GEMM path,
+// k_batch_control, run redundantly and identically in every CTA).
+__device__ void fb_adapt_helper(const FbArgs& a, FbCtl& ctl, FbAdapt& ad, const FbView& u,
+                                int lane) {
+  const int q = lane & 7;
+  auto retire = [&](int c) {
+    const int id = ctl.id[c][q];
+    ad.ret[c][q] = 1;
+    if (u.idx == 0) {
+      a.nacc[id] = ad.cnt[c][0][q];
+      a.nrej[id] = ad.cnt[c][1][q];
+      a.tf[id] = ctl.t[c][q];
+      a.gave_up[id] = ad.done[c][q] == 2;
+    }
+  };
+  // the attempt's step (capped at the time left), its fields, who is left
+  auto prepare = [&](int c, int att) {
+    if (lane < CP) {
+      double hatt = 0.0;
+      if (!ad.done[c][q]) {
+        hatt = ad.h[c][q];
+        const double rem = ad.t_end[c][q] - ctl.t[c][q];
+        ad.lastst[c][q] = hatt >= rem;
+        if (hatt >= rem) hatt = rem;
+      }
+      ad.hatt[c][q] = hatt;
+    }
+    __syncwarp();
+    for (int s = lane >> 3; s < kNumStages; s += 4) {
+      const int id = ctl.id[c][q];
+      ad.F[c][s][q] =
+          ad.done[c][q] ? 0.0 : dev_field(a.pulse[id], ctl.t[c][q] + f_C[s] * ad.hatt[c][q]);
+    }
+    const bool any = __any_sync(0xffffffffu, ad.done[c][q] == 0);
+    if (lane == 0) ad.alive[c] = any;
+    __syncwarp();
+    __threadfence_block();
+    if (lane == 0) ctl.step[c] = att;
+  };
+  for (int c = 0; c < u.nc; ++c) {
+    if (lane < CP) {
+      const int id = ctl.id[c][q];
+      ctl.nrm[c][q] = make_double2(1.0, 1.0);
+      ad.acc[c][q] = ad.ret[c][q] = 0;
+      ad.cnt[c][0][q] = ad.cnt[c][1][q] = ad.cnt[c][2][q] = 0;
+      ad.h[c][q] = a.h0;
+      ctl.t[c][q] = id >= 0 ? a.t0[id] : 0.0;
+      ad.t_end[c][q] = id >= 0 ? a.t_end[id] : 0.0;
+      ad.done[c][q] = id < 0 ? 3 : ctl.t[c][q] >= ad.t_end[c][q] ? 1 : 0;
+      if (ad.done[c][q] == 1) retire(c);
+    }
+    __syncwarp();
+    prepare(c, 0);
+  }
+  unsigned live = 0;
+  for (int c = 0; c < u.nc; ++c)
+    if (ad.alive[c]) live |= 1u << c;
+  int events = 0;
+  for (int n = 0; live; ++n)
+    for (unsigned todo = live; todo; todo &= todo - 1) {
+      const int c = __ffs(todo) - 1;
+      if (!fb_progress(ctl, ++events)) return;
+      const int gc = c * a.ng + u.grp;
+      bool ok = true;
+      if (n > 0)
+        ok = fb_count(a.ctr + gc, (unsigned long long)n * a.gp + a.bc.skew, lane, a.bc.wait_ns);
+      double sum = 0.0, em = 0.0;
+      const double* pp = a.part + ((long long)gc * 2 + (n & 1)) * a.gp * (2 * CP);
+      for (int b0 = lane >> 3; ok && b0 < a.gp; b0 += 16) {
+        double v[4], w[4];
+        unsigned long long t0 = 0;
+        for (unsigned i = 0;; ++i) {
+          bool ready = true;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const bool in = b0 + 4 * j < a.gp;
+            v[j] = in ? ld_relaxed1(pp + (b0 + 4 * j) * (2 * CP) + q) : 0.0;
+            w[j] = in ? ld_relaxed1(pp + (b0 + 4 * j) * (2 * CP) + CP + q) : 0.0;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ready = ready && !is_empty(v[j]) && !is_empty(w[j]);
+          if (ready) break;
+          if ((i & 255u) == 255u) {
+            const unsigned long long t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > a.bc.wait_ns) {
+              ok = false;
+              break;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sum += v[j];
+          em = fb_nanmax(em, w[j]);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) {
+          atomicOr(a.status, ST_WAIT_TIMEOUT);
+          ctl.hdead = 1;
+        }
+        return;
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      em = fb_nanmax(em, __shfl_xor_sync(0xffffffffu, em, 8));
+      em = fb_nanmax(em, __shfl_xor_sync(0xffffffffu, em, 16));
+      if (lane < CP) {
+        ad.acc[c][q] = ad.ret[c][q] = 0;
+        if (!ad.done[c][q]) {
+          const double nrm = sqrt(sum), hh = ad.hatt[c][q];
+          double fac = 5.0;
+          if (em != 0.0) fac = fmin(fmax(0.9 / sqrt(sqrt(sqrt(em))), 0.2), 5.0);
+          ++ad.cnt[c][2][q];
+          if (em <= 1.0 && nrm > 0.0 && isfinite(nrm)) {
+            ctl.t[c][q] = ad.lastst[c][q] ? ad.t_end[c][q] : ctl.t[c][q] + hh;
+            ++ad.cnt[c][0][q];
+            ad.acc[c][q] = 1;
+            ctl.nrm[c][q] = make_double2(nrm, 1.0 / nrm);
+            ad.h[c][q] = fmin(hh * fac, a.dt_max);
+            if (ad.lastst[c][q]) ad.done[c][q] = 1;
+          } else {
+            ++ad.cnt[c][1][q];
+            ad.h[c][q] = hh * fmin(fac, 1.0);
+          }
+          if (!ad.done[c][q] &&
+              (ad.cnt[c][2][q] >= a.max_attempts ||
+               ad.h[c][q] < 1e-13 * fmax(1.0, fabs(ad.t_end[c][q]))))
+            ad.done[c][q] = 2;
+          if (ad.done[c][q]) retire(c);
+        }
+        double* mine = a.part + (((long long)gc * 2 + ((n + 1) & 1)) * a.gp + u.idx) * (2 * CP) + q;
+        st_relaxed1(mine, __longlong_as_double((long long)kEmpty));
+        st_relaxed1(mine + CP, __longlong_as_double((long long)kEmpty));
+      }
+      __syncwarp();
+      prepare(c, n + 1);
+      if (!ad.alive[c]) {
+        live &= ~(1u << c);
+        continue;
+      }
+      // every CTA is past attempt n of this chunk
+      double2* base = a.V + u.cpitch * gc + (long long)u.row0 * CP;
+      const int ne = u.nrows * CP;
+      for (int s = 0; s < kNumStages; ++s) {
+        double2* d = base + u.spitch * ada_y(n, s);
+        for (int e = lane; e < ne; e += 32) st_relaxed2(d + e, empty2());
+      }
+      __syncwarp();
+      if (lane == 0) fb_arrive(a.ctr + gc);
+    }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constant__ FbArgs a) {
   extern __shared__ __align__(16) unsigned char bsm[];
   const FbCta me = a.cta[blockIdx.x];
   FbCtl& ctl = *reinterpret_cast<FbCtl*>(bsm);
   double2* red = reinterpret_cast<double2*>(bsm + (sizeof(FbCtl) + 15) / 16 * 16);
-  __shared__ double red8[FW][CP];
+  // mode 1: the control's second part, then the slopes if they fit
+  FbAdapt& ad = *reinterpret_cast<FbAdapt*>(red + 2 * FW * a.mt * 64);
+  double2* kshm = MODE == 1 && !a.kst
+                      ? reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(&ad) +
+                                                   (sizeof(FbAdapt) + 15) / 16 * 16)
+                      : nullptr;
+  __shared__ double red8[FW][CP], rede[FW][CP];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   FbView u;
   u.w = flow_window(a.g, me.L);
@@ -739,6 +1090,8 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constan
     if (warp == FW) {
       if constexpr (MODE == 2)
         fb_adj_helper(a, ctl, u, lane);
+      else if constexpr (MODE == 1)
+        fb_adapt_helper(a, ctl, ad, u, lane);
       else
         fb_fixed_helper(a, ctl, u, lane);
     }
@@ -748,6 +1101,7 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constan
 #define FB_RUN(I, MT, KT) \
   case I: \
     if constexpr (MODE == 2) fb_adj_main<MT, KT>(a, ctl, u, red, red8, tid); \
+    else if constexpr (MODE == 1) fb_adapt_main<MT, KT>(a, ctl, ad, u, red, kshm, red8, rede, tid); \
     else fb_fixed_main<MT, KT>(a, ctl, u, red, red8, tid); \
     break;
   switch (me.cfg) { FB_CONFIGS(FB_RUN) }
@@ -755,9 +1109,15 @@ __global__ void __launch_bounds__(FTHREADS, 1) k_flow_batch(const __grid_constan
   if (tid == 0) ctl.mexit = 1;
 }
 
-// Shared memory of a CTA: control and two buffers of partial sums.
-inline size_t flowb_smem() {
-  return (sizeof(FbCtl) + 15) / 16 * 16 + sizeof(double2) * 2 * FW * kMaxMT * 64;
+// Shared memory of a launch whose CTAs have at most mt 8-row tiles: control, two
+// buffers of partial sums, and for adaptive steps their control and, where
+// they fit, the slopes of all a group's chunks (`rows` rows per CTA).  The
+// slopes are read up to nine times per item: from shared memory an attempt of 48
+// pulses on 1752 states takes 173 us, from global memory 188.
+inline size_t flowb_smem(int mode, int mt, int slope_chunks = 0, int rows = 0) {
+  return (sizeof(FbCtl) + 15) / 16 * 16 + sizeof(double2) * 2 * FW * mt * 64 +
+         (mode == 1 ? (sizeof(FbAdapt) + 15) / 16 * 16 : 0) +
+         sizeof(double2) * (kNumStages - 1) * (size_t)slope_chunks * rows * CP;
 }
 
 }  // namespace mpc

@@ -79,3 +79,31 @@ def test_gradient_matches_single_pulse(n, B, gauge):
                 assert abs(J[b] - j) < 4e-12
                 assert np.max(np.abs(Fb[b] - f)) <= 1e-11 * max(np.max(np.abs(f)), 1e-3)
                 assert np.max(np.abs(G[b] - g)) <= 1e-11 * max(np.max(np.abs(g)), 1e-3)
+
+
+@pytest.mark.parametrize("gauge", ["l", "v"])
+@pytest.mark.parametrize("B", [1, 9, 20])
+@pytest.mark.parametrize("n", [[1, 1], [60, 70, 50], [97] * 5, [201] * 8, [5, 500, 7]],
+                         ids=lambda n: f"{len(n)}x{max(n)}")
+def test_adaptive_steps_match_stage_gemm(n, B, gauge):
+    """Against the stage-GEMM path (the same controller on other sums): the
+    same accepted and rejected steps and end times; states within 1e-9, ten
+    times the local tolerance of 1e-10, since the step sizes follow an error
+    estimate that is itself rounding noise of the slopes.  A pulse with nothing
+    to do comes back as it went in."""
+    s, pulses, X = _case(n, gauge, B)
+    t0 = 0.3 * np.arange(B)
+    t_end = t0 + 0.8 + 0.1 * (np.arange(B) % 9)
+    if B > 1:
+        t_end[1] = t0[1]
+    out = []
+    for path in ("auto", "streaming"):
+        with mpc_tdse.Context.from_system(s) as ctx:
+            ctx.set_path(path)
+            out.append(ctx.batch_propagate(pulses, t0, t_end, X, dt_max=0.2))
+    (Y, acc, rej, tf), (Z, acc2, rej2, tf2) = out
+    assert np.array_equal(tf, tf2) and np.array_equal(tf, t_end)
+    assert np.array_equal(acc, acc2) and np.array_equal(rej, rej2)
+    assert np.max(np.abs(Y - Z)) < 1e-9
+    if B > 1:
+        assert np.array_equal(Y[1], X[1]) and acc[1] == 0
