@@ -55,10 +55,8 @@ struct ControlArgs {
   FixedStep fx;               // fixed-step mode (the reference's semantics)
   unsigned* status;
   // fixed-step mode: the step's unnormalised x_new [n][ldc] (the next step's
-  // first product normalises it); a pulse that finishes is written out here
+  // first product normalises it)
   const double2* XN;
-  double2* out;               // [B][n] final states (user layout)
-  int ntot;
 };
 
 // The next attempt's step: h capped at the time left (the final step lands
@@ -106,12 +104,18 @@ __global__ void k_batch_control(const __grid_constant__ ControlArgs a) {
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) / kCtlLanes;
   const int lane = threadIdx.x % kCtlLanes;
   const ColState& c = a.c;
+  // ||x_new||^2: the pulse's 16 lanes stride the row tiles' partials (one lane
+  // alone took 11 us at 30 row tiles and 23 at 188), then a fixed xor tree
+  double ns = 0.0;
+  if (q < a.ncol && a.mode != 0)
+    for (int r = lane; r < a.nrowtiles; r += kCtlLanes) ns += a.normpart[(long long)r * a.ldc + q];
+  for (int o = kCtlLanes / 2; o > 0; o >>= 1) ns += __shfl_xor_sync(0xffffffffu, ns, o);
   if (q < a.ncol && lane == 0 && a.fx.on) {
     // fixed-step mode: accept every step whose norm is finite, t += dt as the
     // reference's loop does, retire after nsteps steps.  The state stays
     // unnormalised in XN with its norm in c.nrm (the next step's first
-    // product divides); the _pop entry and a finished pulse's final state are
-    // formed here, dividing as the reference's c /= ||c|| does.
+    // product divides); the _pop entry is formed here, dividing as the
+    // reference's c /= ||c|| does (k_batch_out writes a finished pulse's state).
     c.retired[q] = 0;
     if (a.mode == 0) {
       c.h[q] = a.fx.dt;
@@ -125,8 +129,6 @@ __global__ void k_batch_control(const __grid_constant__ ControlArgs a) {
       c.accepted[q] = 0;
       if (!c.done[q]) {
         a.err[q] = 0ull;
-        double ns = 0.0;
-        for (int r = 0; r < a.nrowtiles; ++r) ns += a.normpart[(long long)r * a.ldc + q];
         const double nrm = sqrt(ns);
         c.natt[q] += 1;
         if (nrm > 0.0 && isfinite(nrm)) {
@@ -165,8 +167,6 @@ __global__ void k_batch_control(const __grid_constant__ ControlArgs a) {
       if (!c.done[q]) {
         const double err = __longlong_as_double((long long)a.err[q]);
         a.err[q] = 0ull;
-        double ns = 0.0;
-        for (int r = 0; r < a.nrowtiles; ++r) ns += a.normpart[(long long)r * a.ldc + q];
         const double nrm = sqrt(ns);
         const double hh = c.hatt[q];
         const double safety = 0.9, facmin = 0.2, facmax = 5.0;
@@ -203,21 +203,28 @@ __global__ void k_batch_control(const __grid_constant__ ControlArgs a) {
     }
   }
   __syncthreads();
-  if (a.fx.on && q < a.ncol && c.retired[q]) {
-    // fixed-step mode: the finished pulse's final state out, by its lanes
-    const double nrm = c.nrm[q];
-    const long long id = c.pulse_id[q];
-    for (int i = lane; i < a.ntot; i += kCtlLanes) {
-      const double2 v = a.XN[(long long)i * a.ldc + q];
-      a.out[id * a.ntot + i] = make_double2(v.x / nrm, v.y / nrm);
-    }
-  }
   if (q < a.ncol && lane < kNumStages) {
     // stage fields F(t + c_s h); in fixed-step mode F(t + dt) for every stage
     const double ts = a.fx.on ? c.t[q] + a.fx.dt : c.t[q] + c_C[lane] * c.hatt[q];
     const double F = c.done[q] ? 0.0 : dev_field(c.pulse[q], ts);
     a.Fs[lane * a.ldc + q] = F;
   }
+}
+
+// Fixed-step mode: the final states of the pulses that have just finished.  The
+// host knows after which steps some do, and launches this there (written by
+// the controller's 16 lanes per pulse it took 90 us at 1752 states and 550 us
+// at 11,914).
+__global__ void k_batch_out(const double2* XN, const int* retired, const double* nrm,
+                            const int* pulse_id, double2* out, int ntot, int ncol, int ldc) {
+  pdl_trigger();
+  pdl_wait();
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (long long)ntot * ncol) return;
+  const int i = (int)(e / ncol), q = (int)(e % ncol);
+  if (!retired[q]) return;
+  const double2 v = XN[(long long)i * ldc + q];
+  out[(long long)pulse_id[q] * ntot + i] = make_double2(v.x / nrm[q], v.y / nrm[q]);
 }
 
 struct ApplyArgs {
@@ -298,10 +305,47 @@ __global__ void k_batch_store_k0(double2* out, const double2* K, int ntot, int n
   out[(long long)q * ntot + i] = K[(long long)i * ldc + q];
 }
 
+// The active columns' scalars to the front, in place, all arrays in one launch
+// of one CTA: map is increasing and map[q] >= q, so what a pass of blockDim
+// columns writes no later pass reads.
 template <class T>
-__global__ void k_gather_scalar(T* dst, const T* src, const int* map, int n) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) dst[q] = src[map[q]];
+__device__ void gather_front(T* v, const int* map, int n) {
+  for (int q0 = 0; q0 < n; q0 += blockDim.x) {
+    const int q = q0 + threadIdx.x;
+    T t{};
+    if (q < n) t = v[map[q]];
+    __syncthreads();
+    if (q < n) v[q] = t;
+    __syncthreads();
+  }
+}
+__global__ void k_batch_compact(ColState c, double* Fs, int ldc, const int* map, int n) {
+  gather_front(c.pulse, map, n);
+  gather_front(c.t, map, n);
+  gather_front(c.t_end, map, n);
+  gather_front(c.h, map, n);
+  gather_front(c.hatt, map, n);
+  gather_front(c.last, map, n);
+  gather_front(c.done, map, n);
+  gather_front(c.accepted, map, n);
+  gather_front(c.nacc, map, n);
+  gather_front(c.nrej, map, n);
+  gather_front(c.natt, map, n);
+  gather_front(c.pulse_id, map, n);
+  gather_front(c.nrm, map, n);
+  gather_front(c.retired, map, n);
+  gather_front(c.nsteps, map, n);
+  for (int s = 0; s < kNumStages; ++s) gather_front(Fs + (long long)s * ldc, map, n);
+}
+
+// Normalised states out of the columns, in the user layout by pulse.
+__global__ void k_batch_states(double2* dst, const double2* XN, const double* nrm,
+                               const int* pulse_id, int ntot, int ncol, int ldc) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (long long)ntot * ncol) return;
+  const int i = (int)(e / ncol), q = (int)(e % ncol);
+  const double2 v = XN[(long long)i * ldc + q];
+  dst[(long long)pulse_id[q] * ntot + i] = make_double2(v.x / nrm[q], v.y / nrm[q]);
 }
 
 }  // namespace
@@ -321,14 +365,17 @@ struct mpc_batch_state {
   int* cnt = nullptr;       // split-variant arrival counters (kept at zero)
   unsigned* hcnt = nullptr; // persistent Horner launch: ticket + per-column progress
   size_t hcnt_n = 0;
-  void* scratch = nullptr;  // compaction staging for per-column scalars
   ColState c{};
   PulseResults res{};
   std::vector<void*> allocs;
-  // autotuned stage-GEMM variant per width bucket (bucket j: up to 2^j pulses)
+  // autotuned stage-GEMM variant per width bucket (bucket j: up to 2^j pulses;
+  // -1: not tuned)
   std::vector<int> tile;
   std::vector<double> tile_us;
-  // fixed-step steps, per width bucket: -1 one launch per Horner product
+  // steps (attempts) run or planned per bucket: a bucket is tuned once there
+  // are kTuneSteps of them, since timing the variants costs about 70 steps
+  std::vector<long long> used_fixed, used_adaptive;
+  // fixed-step steps, per width bucket: kPlanUntuned, -1 one launch per Horner product
   // (on the right-hand-side tuner's variant), kPlanPerProduct + v one launch
   // per product on variant v, v >= 0 the persistent launch on variant v,
   // kPlanTma + s one TMA-fed launch per product on TMA shape s;
@@ -342,6 +389,8 @@ struct mpc_batch_state {
 };
 
 namespace {
+constexpr int kPlanUntuned = -2;
+constexpr long long kTuneSteps = 200;
 constexpr int kPlanTma = 100;
 constexpr int kPlanPerProduct = 200;
 }
@@ -383,7 +432,6 @@ int ensure_batch(mpc_ctx* c, int B) {
       (rc = balloc(b, &b->ws, split_ws_doubles(nrt, ldc))) ||
       (rc = balloc(b, &b->cnt, split_cnt_ints(nrt, ldc))) ||
       (rc = balloc(b, &b->hcnt, 1 + 12 * (size_t)((2 * ldc + 15) / 16) * kMaxBlocks)) ||
-      (rc = balloc(b, reinterpret_cast<char**>(&b->scratch), sizeof(mpc_pulse) * ldc)) ||
       (rc = balloc(b, &s.pulse, ldc)) || (rc = balloc(b, &s.t, ldc)) ||
       (rc = balloc(b, &s.t_end, ldc)) || (rc = balloc(b, &s.h, ldc)) ||
       (rc = balloc(b, &s.hatt, ldc)) || (rc = balloc(b, &s.last, ldc)) ||
@@ -470,8 +518,8 @@ int launch_stage(mpc_ctx* c, const StageArgs& a) {
 
 // How a fixed step of ncol pulses runs: -1 one launch per Horner product,
 // else the persistent launch (k_batch_horner) on tile variant v.  The
-// fixed-step tuner's choice when it ran; otherwise persistent on the tuned
-// variant when a product has enough tiles to fill the GPU.
+// fixed-step tuner's choice when it ran, otherwise the default for the number
+// of tiles.
 int horner_plan(mpc_ctx* c, int ncol) {
   if (c->no_persist) return -1;
   const mpc_batch_state* b = c->batch;
@@ -480,11 +528,9 @@ int horner_plan(mpc_ctx* c, int ncol) {
   if (c->forced_variant >= 0 && c->forced_variant < kNumVariants)
     return kPlanPerProduct + c->forced_variant;
   const int j = width_bucket(ncol);
-  if (j < (int)b->hplan.size()) return b->hplan[j];
-  const int v = mpc_batch_variant(c, ncol);
-  const int bn = horner_tile_bn(v);
-  const int ncolt = (2 * ncol + bn - 1) / bn;
-  return (long long)ncolt * b->nrowtiles >= c->num_sms ? v : -1;
+  if (j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned) return b->hplan[j];
+  const int v = default_variant(ncol, b->nrowtiles);
+  return default_persistent(ncol, b->nrowtiles) ? v : kPlanPerProduct + v;
 }
 
 
@@ -579,106 +625,108 @@ long long horner_step_launches(mpc_ctx* c, int ncol) {
   return (plan >= 0 && plan < kPlanTma) ? 2 : 13;
 }
 
-// Times every variant on a single right-hand side (stage 0, k only) at
-// widths 1, 2, 4, ... up to max_cols pulses and keeps the fastest per width.
-// Every variant sums in the same order, so the choice affects speed only.
-int autotune(mpc_ctx* c, int max_cols) {
+// Times every variant on a single right-hand side (stage 0, k only) at bucket
+// j's width and keeps the fastest.  Every variant sums in the same order, so
+// the choice affects speed only.
+int tune_bucket(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
   mpc_batch_state* b = c->batch;
-  const int top = width_bucket(std::min(std::max(max_cols, 1), b->ldc));
-  std::vector<int> tile(top + 1);
-  std::vector<double> us((size_t)(top + 1) * kNumVariants);
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  int rc = MPC_OK;
-  for (int j = 0; j <= top && rc == MPC_OK; ++j) {
-    const int w = std::min(1 << j, b->ldc);
-    const StageArgs a = stage_args(c, 0, w, 0.0, 0.0, true);
-    double best = 1e300;
-    for (int v = 0; v < kNumVariants && rc == MPC_OK; ++v) {
-      cudaError_t e = cudaSuccess;
-      for (int r = 0; r < 2 && e == cudaSuccess; ++r) e = launch_variant<0>(c->stream, v, a);
-      if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
-      const int reps = 5;
-      for (int r = 0; r < reps && e == cudaSuccess; ++r) e = launch_variant<0>(c->stream, v, a);
-      if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-      float ms = 0.0f;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      if (e != cudaSuccess) {
-        rc = mpc_fail(MPC_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
-        break;
-      }
-      c->launches += 2 + reps;
-      const double t = 1000.0 * ms / reps;
-      us[(size_t)j * kNumVariants + v] = t;
-      if (t < best) {
-        best = t;
-        tile[j] = v;
-      }
+  if ((int)b->tile.size() <= j) {
+    b->tile.resize(j + 1, -1);
+    b->tile_us.resize((size_t)(j + 1) * kNumVariants, 0.0);
+  }
+  const StageArgs a = stage_args(c, 0, std::min(1 << j, b->ldc), 0.0, 0.0, true);
+  double best = 1e300;
+  for (int v = 0; v < kNumVariants; ++v) {
+    const int reps = 5;
+    for (int r = 0; r < 2; ++r) CK(launch_variant<0>(c->stream, v, a));
+    CK(cudaEventRecord(e0, c->stream));
+    for (int r = 0; r < reps; ++r) CK(launch_variant<0>(c->stream, v, a));
+    CK(cudaEventRecord(e1, c->stream));
+    CK(cudaEventSynchronize(e1));
+    float ms = 0.0f;
+    CK(cudaEventElapsedTime(&ms, e0, e1));
+    c->launches += 2 + reps;
+    const double t = 1000.0 * ms / reps;
+    b->tile_us[(size_t)j * kNumVariants + v] = t;
+    if (t < best) {
+      best = t;
+      b->tile[j] = v;
     }
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (rc) return rc;
-  b->tile = tile;
-  b->tile_us = us;
   return MPC_OK;
 }
 
-// The fixed-step tuner: at widths 1, 2, 4, ... up to max_cols pulses, times
-// one whole step's 12 Horner products as one launch per product (on the
-// tuned variant) and as the persistent launch on each unsplit tile shape,
-// and keeps the fastest.  Every candidate computes the same tiles in the same
-// order, so the choice changes speed only.  Runs on the batch's work
-// buffers before the propagation loads its states.
-int autotune_horner(mpc_ctx* c, int max_cols) {
+// The fixed-step tuner: times one whole step's 12 Horner products at bucket j's
+// width as one launch per product on every tile variant (the right-hand-side
+// tuner's choice need not suit the Horner epilogue) and as the persistent
+// launch on every unsplit variant, and keeps the fastest.  Every candidate
+// computes the same tiles in the same order, so the choice changes speed only.
+// (The TMA-fed launches are not among them: 720 / 428 / 189 us per step at 256 /
+// 64 / 16 pulses against 616 / 250 / 145.)  Runs on the batch's work buffers,
+// before the propagation loads its states, with unit norms in c.nrm.
+int tune_bucket_fixed(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
   mpc_batch_state* b = c->batch;
-  const int top = width_bucket(std::min(std::max(max_cols, 1), b->ldc));
-  std::vector<int> plan(top + 1, -1);
-  std::vector<double> plan_us(top + 1, 0.0);
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  // one launch per product on every tile variant (the right-hand-side
-  // tuner's choice need not suit the Horner epilogue), the persistent launch
-  // on every unsplit variant, the TMA-fed launches
+  if ((int)b->hplan.size() <= j) {
+    b->hplan.resize(j + 1, kPlanUntuned);
+    b->hplan_us.resize(j + 1, 0.0);
+  }
   std::vector<int> cands = {0, 1, 2, 3, 4};
   for (int v = 0; v < kNumVariants; ++v) cands.push_back(kPlanPerProduct + v);
-  if (b->tma_ok && !c->no_tma)
-    for (int sh = 0; sh < kNumTmaShapes; ++sh) cands.push_back(kPlanTma + sh);
-  int rc = MPC_OK;
   const long long l0 = c->launches;
-  for (int j = 0; j <= top && rc == MPC_OK; ++j) {
-    const int w = std::min(1 << j, b->ldc);
-    double best = 1e300;
-    for (int v : cands) {
-      auto step = [&]() -> int { return launch_horner_plan(c, w, v); };
-      for (int r = 0; r < 2 && rc == MPC_OK; ++r) rc = step();
-      if (rc) break;
+  const int w = std::min(1 << j, b->ldc);
+  double best = 1e300;
+  int rc;
+  for (int v : cands) {
+    double t = 0.0;
+    for (int pass = 0; pass < 2; ++pass) {   // the first one warms up, and drops the slow
+      const int reps = pass ? 3 : 1;
       CK(cudaEventRecord(e0, c->stream));
-      const int reps = 3;
-      for (int r = 0; r < reps && rc == MPC_OK; ++r) rc = step();
-      if (rc) break;
+      for (int r = 0; r < reps; ++r)
+        if ((rc = launch_horner_plan(c, w, v))) return rc;
       CK(cudaEventRecord(e1, c->stream));
       CK(cudaEventSynchronize(e1));
       float ms = 0.0f;
       CK(cudaEventElapsedTime(&ms, e0, e1));
-      const double t = 1000.0 * ms / reps;
-      if (t < best) {
-        best = t;
-        plan[j] = v;
-        plan_us[j] = t;
-      }
+      t = 1000.0 * ms / reps;
+      if (t > 2.0 * best) break;
+    }
+    if (t < best) {
+      best = t;
+      b->hplan[j] = v;
+      b->hplan_us[j] = t;
     }
   }
   c->launches = l0;
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (rc) return rc;
-  b->hplan = plan;
-  b->hplan_us = plan_us;
   return MPC_OK;
+}
+
+// Tunes what a call is about to use: every bucket whose steps, run so far and
+// planned[j] now, reach kTuneSteps (all: whatever they are).
+int tune(mpc_ctx* c, bool fixed, const std::vector<long long>& planned, bool all) {
+  mpc_batch_state* b = c->batch;
+  std::vector<long long>& used = fixed ? b->used_fixed : b->used_adaptive;
+  if (used.size() < planned.size()) used.resize(planned.size(), 0);
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  int rc = MPC_OK;
+  for (int j = 0; j < (int)planned.size() && rc == MPC_OK; ++j) {
+    used[j] += planned[j];
+    const bool have = fixed ? j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned
+                            : j < (int)b->tile.size() && b->tile[j] >= 0;
+    if (have || (!all && (planned[j] == 0 || used[j] < kTuneSteps))) continue;
+    if (!e0) {
+      CK(cudaEventCreate(&e0));
+      CK(cudaEventCreate(&e1));
+      if (fixed) {   // the first product divides by the columns' norms
+        std::vector<double> ones(b->ldc, 1.0);
+        CK(cudaMemcpyAsync(b->c.nrm, ones.data(), sizeof(double) * b->ldc, cudaMemcpyHostToDevice,
+                           c->stream));
+      }
+    }
+    rc = fixed ? tune_bucket_fixed(c, j, e0, e1) : tune_bucket(c, j, e0, e1);
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  return rc;
 }
 
 }  // namespace
@@ -688,9 +736,12 @@ int mpc_batch_variant(mpc_ctx* c, int ncol) {
   if (c->batch) {
     const std::vector<int>& t = c->batch->tile;
     const int j = width_bucket(ncol);
-    if (j < (int)t.size()) return t[j];
+    if (j < (int)t.size() && t[j] >= 0) return t[j];
   }
-  return default_variant(ncol);
+  int nrt = 0;
+  for (int L = 0; L < c->g.nstate_blk; ++L)
+    nrt += (c->g.state_off[L + 1] - c->g.state_off[L] + BM - 1) / BM;
+  return default_variant(ncol, nrt);
 }
 
 void mpc_batch_free(mpc_ctx* c) {
@@ -746,8 +797,9 @@ int mpc_batch_fixed_plan(mpc_ctx* c, double* table, int cap) {
   const mpc_batch_state* b = c->batch;
   const int rows = (int)b->hplan.size();
   for (int j = 0; table && j < rows && j < cap; ++j) {
-    const int v = b->hplan[j];
+    int v = b->hplan[j];
     table[5 * j + 0] = std::min(1 << j, b->ldc);
+    if (v == kPlanUntuned) v = horner_plan(c, std::min(1 << j, b->ldc));
     if (v >= kPlanPerProduct) {
       const TileVariant& tv = kVariants[v - kPlanPerProduct];
       table[5 * j + 1] = tv.split ? 3 : 0;
@@ -773,7 +825,7 @@ int mpc_batch_autotune(mpc_ctx* c, int B, double* table, int cap) {
   CK(cudaSetDevice(c->device));
   int rc;
   if ((rc = ensure_batch(c, B))) return rc;
-  if ((rc = autotune(c, B))) return rc;
+  if ((rc = tune(c, false, std::vector<long long>(width_bucket(B) + 1, 0), true))) return rc;
   const mpc_batch_state* b = c->batch;
   const int rows = (int)b->tile.size();
   for (int j = 0; table && j < rows && j < cap; ++j) {
@@ -807,15 +859,24 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
 
   if (fx.on && c->force_tma > 0 && !b->tma_ok)
     return mpc_fail(MPC_ERR_CUDA, "MPC_FORCE_TMA: the TMA tensor maps could not be set up");
-  // the fixed-step tuner times Horner steps on the work buffers (the first
-  // product writes X): it runs before the states are loaded, on unit norms
-  if (b->tile.empty() && !std::getenv("MPC_NO_AUTOTUNE") && (rc = autotune(c, B))) return rc;
-  if (fx.on && b->hplan.empty() && !c->no_persist && !c->force_persist && !c->force_tma &&
-      !std::getenv("MPC_NO_AUTOTUNE")) {
-    std::vector<double> ones(ldc, 1.0);
-    CK(cudaMemcpyAsync(s.nrm, ones.data(), sizeof(double) * ldc, cudaMemcpyHostToDevice,
-                       c->stream));
-    if ((rc = autotune_horner(c, B))) return rc;
+  // the tuners run on the work buffers, before the states are loaded; what each
+  // width is about to run is known for fixed steps, and bounded from below by
+  // the longest pulse's steps of dt_max for adaptive ones
+  if (!std::getenv("MPC_NO_AUTOTUNE") &&
+      !(fx.on && (c->no_persist || c->force_persist || c->force_tma))) {
+    std::vector<long long> planned(width_bucket(B) + 1, 0);
+    if (fx.on) {
+      std::vector<int> len(nsteps, nsteps + B);
+      std::sort(len.begin(), len.end());
+      for (int k = 0; k < B; ++k)   // B - k pulses run the steps (len[k-1], len[k]]
+        if (!mpc_flowb_wanted(c, B - k))
+          planned[width_bucket(B - k)] += len[k] - (k ? len[k - 1] : 0);
+    } else {
+      double most = 0.0;
+      for (int k = 0; k < B; ++k) most = std::max(most, t_end[k] - t0[k]);
+      planned.back() = (long long)std::min(most / dt_max, 1e6);
+    }
+    if ((rc = tune(c, fx.on, planned, false))) return rc;
   }
 
   // per-column start state
@@ -827,6 +888,7 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   CK(cudaMemcpyAsync(s.t_end, t_end, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(s.pulse_id, ids.data(), sizeof(int) * B, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(s.nacc, zeros.data(), sizeof(int) * B, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemsetAsync(b->res.status, 0, sizeof(int) * B, c->stream));
   CK(cudaMemcpyAsync(s.nrej, zeros.data(), sizeof(int) * B, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(s.natt, zeros.data(), sizeof(int) * B, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(s.nsteps, fx.on ? nsteps : zeros.data(), sizeof(int) * B,
@@ -854,8 +916,6 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   ca.fx = fx;
   ca.status = c->d_status;
   ca.XN = b->Y[0];
-  ca.out = b->out;
-  ca.ntot = n;
   ApplyArgs aa{};
   aa.X = b->X;
   aa.Xn = b->Y[1];
@@ -882,6 +942,15 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
     c->launches += 2;
   }
   c->launches += 1;
+  // fixed-step mode: the final states of what has just finished
+  auto states_out = [&]() -> int {
+    CK(mpc_launch_pdl(k_batch_out, dim3(blocks_for((long long)n * ncol, 256)), dim3(256), 0,
+                      c->stream, (const double2*)b->Y[0], (const int*)s.retired,
+                      (const double*)s.nrm, (const int*)s.pulse_id, b->out, n, ncol, ldc));
+    ++c->launches;
+    return MPC_OK;
+  };
+  if (fx.on && (rc = states_out())) return rc;
 
   // Few pulses left on a system whose coupling fits on chip: the persistent
   // resident kernel takes over (unless the streamed path was asked for).
@@ -898,8 +967,18 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   auto width = [](int nc) {
     return 2 * nc <= 16 ? 16 : (2 * nc <= 128 ? (2 * nc + 31) / 32 * 32 : (2 * nc + 63) / 64 * 64);
   };
+  // in fixed-step mode the GEMM path keeps the state unnormalised in Y[0];
+  // the resident tail keeps it normalised in X
+  bool state_in_y0 = fx.on;
   // active columns -> map_h[0 .. act)
   auto scan = [&](int* act) -> int {
+    if (fx.on && state_in_y0) {   // every pulse's steps are known: no need to ask
+      int k = 0;
+      for (int q = 0; q < ncol; ++q)
+        if (steps_h[colpid[q]] > steps_done) map_h[k++] = q;
+      *act = k;
+      return MPC_OK;
+    }
     CK(cudaMemcpyAsync(done_h.data(), s.done, sizeof(int) * ncol, cudaMemcpyDeviceToHost,
                        c->stream));
     unsigned st = 0;
@@ -917,10 +996,8 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   };
   // Compaction: the active columns move to the front of X and of every
   // per-column array (the results of retired pulses are already out).
-  // (in fixed-step mode the GEMM path keeps the state unnormalised in Y[0];
-  // the resident tail keeps it normalised in X)
-  bool state_in_y0 = fx.on;
   auto compact = [&](int act) -> int {
+    // (pageable: copied before the call returns)
     CK(cudaMemcpyAsync(b->map, map_h.data(), sizeof(int) * act, cudaMemcpyHostToDevice,
                        c->stream));
     const int gb = blocks_for((long long)n * act, 256);
@@ -933,40 +1010,14 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
       CK(cudaMemcpyAsync(b->X, b->Y[0], sizeof(double2) * (size_t)n * ldc,
                          cudaMemcpyDeviceToDevice, c->stream));
     }
-    const int sb = blocks_for(act, 128);
-#define GATHER(field, T)                                                                    \
-  k_gather_scalar<T><<<sb, 128, 0, c->stream>>>(reinterpret_cast<T*>(b->scratch), s.field,  \
-                                               b->map, act);                               \
-  CK(cudaMemcpyAsync(s.field, b->scratch, sizeof(T) * act, cudaMemcpyDeviceToDevice, c->stream));
-    GATHER(pulse, mpc_pulse)
-    GATHER(t, double)
-    GATHER(t_end, double)
-    GATHER(h, double)
-    GATHER(hatt, double)
-    GATHER(last, int)
-    GATHER(done, int)
-    GATHER(accepted, int)
-    GATHER(nacc, int)
-    GATHER(nrej, int)
-    GATHER(natt, int)
-    GATHER(pulse_id, int)
-    GATHER(nrm, double)
-    GATHER(retired, int)
-    GATHER(nsteps, int)
+    k_batch_compact<<<1, 1024, 0, c->stream>>>(s, b->Fs, ldc, b->map, act);
     {
       std::vector<int> cp(act);
       for (int k = 0; k < act; ++k) cp[k] = colpid[map_h[k]];
       std::copy(cp.begin(), cp.end(), colpid.begin());
     }
-    for (int st = 0; st < kNumStages; ++st) {
-      k_gather_scalar<double><<<sb, 128, 0, c->stream>>>(reinterpret_cast<double*>(b->scratch),
-                                                         b->Fs + st * ldc, b->map, act);
-      CK(cudaMemcpyAsync(b->Fs + st * ldc, b->scratch, sizeof(double) * act,
-                         cudaMemcpyDeviceToDevice, c->stream));
-    }
-#undef GATHER
     CK(cudaGetLastError());
-    c->launches += 16;
+    c->launches += 2;
     ncol = act;
     return MPC_OK;
   };
@@ -1014,8 +1065,10 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
     gexec = nullptr;
     g_ncol = -1;
   };
-  auto run_group = [&]() -> int {
-    if (use_graph && g_ncol != ncol) {
+  // (`left` attempts to come at this width: capturing pays from about 64)
+  auto run_group = [&](long long left) -> int {
+    const bool graph = use_graph && (g_ncol == ncol || left >= 64);
+    if (graph && g_ncol != ncol) {
       drop_graph();
       cudaGraph_t graph = nullptr;
       bool ok = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -1034,7 +1087,7 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
         g_ncol = ncol;
       }
     }
-    if (use_graph) {
+    if (graph && use_graph) {
       CK(cudaGraphLaunch(gexec, c->stream));
       c->launches += (fx.on ? horner_step_launches(c, ncol) : 16LL) * check_every;
       return MPC_OK;
@@ -1048,6 +1101,27 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
     int act = 0;
     if ((rc = scan(&act))) break;
     if (act == 0) break;
+    if (fx.on && mpc_flowb_wanted(c, act)) {
+      // the persistent batched kernels are the faster path from here on
+      if (act < ncol && (rc = compact(act))) break;
+      double2* in = nullptr;
+      if ((rc = mpc_flowb_states(c, B, &in))) break;
+      k_batch_states<<<blocks_for((long long)n * ncol, 256), 256, 0, c->stream>>>(
+          in, b->Y[0], s.nrm, s.pulse_id, n, ncol, ldc);
+      CK(cudaGetLastError());
+      ++c->launches;
+      std::vector<int> ids(colpid.begin(), colpid.begin() + ncol), left(B, 0);
+      std::vector<double> tb(t0, t0 + B);
+      for (int id : ids) {
+        left[id] = (int)(steps_h[id] - steps_done);
+        for (long long k = 0; k < steps_done; ++k) tb[id] += fx.dt;   // as the steps added it
+      }
+      FixedStep rest = fx;
+      if (rest.pop_hist) rest.pop_hist += steps_done;
+      if (rest.norm_hist) rest.norm_hist += steps_done;
+      rc = mpc_flowb_tail(c, B, ids, pulses, tb.data(), left.data(), rest, b->out);
+      break;
+    }
     if (pres && act <= pres) {
       if (act < ncol && (rc = compact(act))) break;
       if (fx.on) {  // the resident kernel takes normalised states in X
@@ -1094,14 +1168,14 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
       }
       if (until <= 0) until = 1;
       for (long long k = 0; k + check_every <= until && rc == MPC_OK; k += check_every)
-        rc = run_group();
+        rc = run_group(until - k);
       for (long long k = until - until % check_every; k < until && rc == MPC_OK; ++k)
         rc = launch_attempt();
-      if (rc) break;
+      if (rc || (rc = states_out())) break;
       steps_done += until;
       continue;
     }
-    if ((rc = run_group())) break;
+    if ((rc = run_group(64))) break;
   }
   drop_graph();
   if (rc) return rc;
@@ -1113,6 +1187,13 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   CK(cudaMemcpyAsync(tf.data(), b->res.t, sizeof(double) * B, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(stt.data(), b->res.status, sizeof(int) * B, cudaMemcpyDeviceToHost,
                      c->stream));
+  unsigned status = 0;
+  CK(cudaMemcpyAsync(&status, c->d_status, sizeof status, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (status) {
+    CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+    return mpc_fail(MPC_ERR_DEVICE, "kernel status 0x%x in the batched propagation", status);
+  }
   CK(cudaMemcpyAsync(ct, b->out, sizeof(double2) * (size_t)n * B, cudaMemcpyDeviceToHost,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));

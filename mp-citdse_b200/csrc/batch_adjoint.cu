@@ -32,7 +32,7 @@ using namespace mpc;
 
 namespace {
 
-constexpr int kDotRows = 64;  // rows per partial of a column inner product
+constexpr int kDotRows = 16;  // rows per partial of a column inner product (64: 21 us at 48 pulses)
 
 // [B][n] (user layout) -> [n][ldc]
 __global__ void k_fb_load(double2* X, const double2* in, int ntot, int ncol, int ldc) {
@@ -42,15 +42,22 @@ __global__ void k_fb_load(double2* X, const double2* in, int ntot, int ncol, int
   X[(long long)i * ldc + q] = in[(long long)q * ntot + i];
 }
 
-// per column: ||x_new|| from the stage kernel's row-tile partials, in order
+// Sum of rows 0 .. n-1 of column q of v [n][ldc]: a warp, lanes striding the
+// rows, then a fixed xor tree.
+__device__ __forceinline__ double warp_column_sum(const double* v, int n, int ldc, int q) {
+  double s = 0.0;
+  for (int r = threadIdx.x & 31; r < n; r += 32) s += v[(long long)r * ldc + q];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// per column: ||x_new|| from the stage kernel's row-tile partials (a warp each)
 __global__ void k_fb_norm(const double* normpart, int nrt, int ldc, int ncol, double* nrm) {
   pdl_trigger();
   pdl_wait();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ncol) return;
-  double s = 0.0;
-  for (int r = 0; r < nrt; ++r) s += normpart[(long long)r * ldc + q];
-  nrm[q] = sqrt(s);
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const double s = warp_column_sum(normpart, nrt, ldc, q < ncol ? q : 0);
+  if (q < ncol && (threadIdx.x & 31) == 0) nrm[q] = sqrt(s);
 }
 
 __global__ void k_fb_scale(const double2* XN, const double* nrm, double2* X, int ntot, int ncol,
@@ -99,11 +106,9 @@ __global__ void k_fb_dot(const double2* x, const double2* lam, double* part, int
 __global__ void k_fb_colsum(const double* part, int nchunk, int ldc, int ncol, double* out) {
   pdl_trigger();
   pdl_wait();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ncol) return;
-  double s = 0.0;
-  for (int c = 0; c < nchunk; ++c) s += part[(long long)c * ldc + q];
-  out[q] = s;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const double s = warp_column_sum(part, nchunk, ldc, q < ncol ? q : 0);
+  if (q < ncol && (threadIdx.x & 31) == 0) out[q] = s;
 }
 
 // zbar = (lam - x1 Re<x1, lam>) / ||z_n||; kbar_12 = h b_12 zbar
@@ -123,16 +128,14 @@ __global__ void k_fb_zbar(const double2* lam, const double2* x1, const double* d
   kb12[idx] = make_double2(hb12 * z.x, hb12 * z.y);
 }
 
-// dJ/dF_n per column: stages, then row tiles, in order
+// dJ/dF_n per column: stages and row tiles (a warp per column; one thread each
+// took 121 us at 30 row tiles)
 __global__ void k_fb_fbar(const double* fpart, int nrt, int ldc, int ncol, double* fbar) {
   pdl_trigger();
   pdl_wait();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ncol) return;
-  double s = 0.0;
-  for (int st = 0; st < kNumStages; ++st)
-    for (int r = 0; r < nrt; ++r) s += fpart[((long long)st * nrt + r) * ldc + q];
-  fbar[q] = s;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const double s = warp_column_sum(fpart, kNumStages * nrt, ldc, q < ncol ? q : 0);
+  if (q < ncol && (threadIdx.x & 31) == 0) fbar[q] = s;
 }
 
 }  // namespace
@@ -289,7 +292,7 @@ int fb_step(mpc_ctx* c, int step, const double2* x, double2* ys, double2* x_out,
   }
   const int n = c->g.ntot, B = a->B;
   ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
-  CK(mpc_launch_pdl(k_fb_norm, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
+  CK(mpc_launch_pdl(k_fb_norm, dim3(blocks_for(B, 4)), dim3(128), 0, c->stream,
                     (const double*)a->normpart, a->nrt, a->ldc, B, nrm_out));
   CK(mpc_launch_pdl(k_fb_scale, dim3(blocks_for((long long)n * B, 256)), dim3(256), 0, c->stream,
                     (const double2*)a->XN, (const double*)nrm_out, x_out, n, B, a->ldc));
@@ -537,7 +540,7 @@ int mpc_batch_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
           ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
           CK(mpc_launch_pdl(k_fb_dot, dim3(a->nchunk, blocks_for(B, 64)), dim3(64), 0, c->stream,
                             x1, (const double2*)a->KB[1], a->dpart, n, B, ldc));
-          CK(mpc_launch_pdl(k_fb_colsum, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
+          CK(mpc_launch_pdl(k_fb_colsum, dim3(blocks_for(B, 4)), dim3(128), 0, c->stream,
                             (const double*)a->dpart, a->nchunk, ldc, B, a->dsum));
           CK(mpc_launch_pdl(k_fb_zbar, dim3(eb), dim3(256), 0, c->stream, (const double2*)a->KB[1],
                             x1, (const double*)a->dsum, (const double*)(a->segN + (size_t)j * ldc),
@@ -554,7 +557,7 @@ int mpc_batch_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
         }
         {
           ProfScope ps(c, MPC_KERNEL_BATCH_OTHER);
-          CK(mpc_launch_pdl(k_fb_fbar, dim3(blocks_for(B, 128)), dim3(128), 0, c->stream,
+          CK(mpc_launch_pdl(k_fb_fbar, dim3(blocks_for(B, 4)), dim3(128), 0, c->stream,
                             (const double*)a->fpart, a->nrt, ldc, B, a->fbar + (size_t)stp * ldc));
           ++c->launches;
         }

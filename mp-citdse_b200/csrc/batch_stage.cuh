@@ -941,10 +941,22 @@ inline int width_bucket(int ncol) {
   return j;
 }
 
-// Before tuning: the narrowest tile that covers the pulses.
-inline int default_variant(int ncol) {
-  const int ncr = 2 * ncol;
-  return ncr <= 16 ? 1 : (ncr <= 128 ? 3 : 4);
+// Before tuning: by the number T of 64 x 16 tiles, on 148 SMs with two CTAs
+// each.  The tuner's picks for 12 Horner products on 1752 to 13,200 states (30 to
+// 208 row tiles) and 1 to 256 pulses: the split (twice the CTAs) up to T = 63;
+// whole tiles with the deep ring at 118 to 126; the shallow ring (two CTAs per
+// SM) from 236 to 832; wider tiles from 960, 64 columns from 1504.
+inline int tiles16(int ncol, int nrt) { return nrt * ((2 * ncol + 15) / 16); }
+inline int default_variant(int ncol, int nrt) {
+  const int T = tiles16(ncol, nrt);
+  return T <= 100 ? 5 : T <= 150 ? 1 : T <= 900 ? 0 : T <= 1300 ? 2 : 4;
+}
+// ... and of a whole fixed step: at 188 and 208 tiles (between one and one and
+// a half per SM) and from 960 the persistent launch was faster (1.49 against
+// 1.9 ms at 11,914 states and 4 pulses, 6.17 against 6.6 at 64).
+inline bool default_persistent(int ncol, int nrt) {
+  const int T = tiles16(ncol, nrt);
+  return (T > 150 && T <= 222) || T > 900;
 }
 
 template <int BN, int NST, int MODE, int SPLIT>

@@ -552,50 +552,47 @@ bool mpc_flowb_wanted(mpc_ctx* c, int B) {
   return f->grp[ng].ok && product_us(f->grp[ng].cost, (nch + ng - 1) / ng) <= gemm_us(c->g, B);
 }
 
-// The fixed-step propagation of B pulses (mpc_batch_advance): ct host [B][n]
-// in and out; pop_out / norm_out host, rows of `ld` and ld - 1 (or null).
-int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
-                      const int* steps, int pop_index, double* ct, double* pop_out,
-                      double* norm_out, int max_steps) {
+int mpc_flowb_states(mpc_ctx* c, int B, double2** in) {
   mpc_flowb_state* f = c->flowb;
-  const int n = c->g.ntot;
+  int rc;
+  if ((rc = grow(&f->io, &f->io_n, 2 * (size_t)B * c->g.ntot))) return rc;
+  *in = f->io;
+  return MPC_OK;
+}
+
+int mpc_flowb_tail(mpc_ctx* c, int B, const std::vector<int>& ids, const mpc_pulse* pulses,
+                   const double* t, const int* left, const FixedStep& fx, double2* out) {
+  mpc_flowb_state* f = c->flowb;
   int rc;
   // pulses by length, so that a chunk's end together
-  std::vector<int> order(B);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return steps[x] > steps[y]; });
-  const int nch_all = (B + CP - 1) / CP;
-  const long long ld = (long long)max_steps + 1;
-  const size_t hist = (size_t)B * ld;
+  std::vector<int> order(ids);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return left[x] > left[y]; });
+  const int nch_all = (int)(order.size() + CP - 1) / CP;
   std::vector<int> ints((size_t)nch_all * (CP + 1) + B, -1);
   int* cid = ints.data();
   int* cst = cid + (size_t)nch_all * CP;
   int* ns = cst + nch_all;
-  for (int i = 0; i < B; ++i) cid[i] = order[i];
-  for (int k = 0; k < nch_all; ++k) cst[k] = steps[order[(size_t)k * CP]];
-  std::copy(steps, steps + B, ns);
-  if ((rc = grow(&f->ints, &f->ints_n, ints.size())) || (rc = grow(&f->pulse, &f->pulse_n, (size_t)B)) ||
-      (rc = grow(&f->t0, &f->t0_n, (size_t)B)) || (rc = grow(&f->io, &f->io_n, 2 * (size_t)B * n)) ||
-      (rc = grow(&f->hist, &f->hist_n, (pop_out ? hist : 0) + (norm_out ? hist : 0) + 1)))
+  std::copy(order.begin(), order.end(), cid);
+  for (int k = 0; k < nch_all; ++k) cst[k] = left[order[(size_t)k * CP]];
+  std::copy(left, left + B, ns);
+  if ((rc = grow(&f->ints, &f->ints_n, ints.size())) ||
+      (rc = grow(&f->pulse, &f->pulse_n, (size_t)B)) || (rc = grow(&f->t0, &f->t0_n, (size_t)B)))
     return rc;
-  double2* in = f->io;
-  double2* out = f->io + (size_t)B * n;
-  CK(cudaMemcpyAsync(in, ct, sizeof(double2) * (size_t)B * n, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(f->ints, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaMemcpyAsync(f->pulse, pulses, sizeof(mpc_pulse) * B, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(f->t0, t0, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(f->t0, t, sizeof(double) * B, cudaMemcpyHostToDevice, c->stream));
   FbArgs a{};
-  a.in = in;
+  a.in = f->io;
   a.out = out;
   a.pulse = f->pulse;
   a.t0 = f->t0;
   a.nsteps = f->ints + (ns - cid);
-  a.dt = dt;
-  a.pop_index = pop_index;
-  a.hist_ld = ld;
-  a.pop_hist = pop_out ? f->hist : nullptr;
-  a.norm_hist = norm_out ? f->hist + (pop_out ? hist : 0) : nullptr;
+  a.dt = fx.dt;
+  a.pop_index = fx.pop_index;
+  a.hist_ld = fx.hist_ld;
+  a.pop_hist = fx.pop_hist;
+  a.norm_hist = fx.norm_hist;
   // launches of at most kMaxChunks chunks per column group
   for (int k0 = 0; k0 < nch_all;) {
     const int ng = pick_groups(f, nch_all - k0);
@@ -605,6 +602,35 @@ int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
     if ((rc = launch(c, a, ng, nch, 0))) return rc;
     k0 += nch;
   }
+  CK(cudaStreamSynchronize(c->stream));   // the host arrays go away
+  return MPC_OK;
+}
+
+// The fixed-step propagation of B pulses (mpc_batch_advance): ct host [B][n]
+// in and out; pop_out / norm_out host, rows of `ld` and ld - 1 (or null).
+int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
+                      const int* steps, int pop_index, double* ct, double* pop_out,
+                      double* norm_out, int max_steps) {
+  mpc_flowb_state* f = c->flowb;
+  const int n = c->g.ntot;
+  int rc;
+  const long long ld = (long long)max_steps + 1;
+  const size_t hist = (size_t)B * ld;
+  double2* in = nullptr;
+  if ((rc = mpc_flowb_states(c, B, &in)) ||
+      (rc = grow(&f->hist, &f->hist_n, (pop_out ? hist : 0) + (norm_out ? hist : 0) + 1)))
+    return rc;
+  double2* out = in + (size_t)B * n;
+  CK(cudaMemcpyAsync(in, ct, sizeof(double2) * (size_t)B * n, cudaMemcpyHostToDevice, c->stream));
+  FixedStep fx{};
+  fx.dt = dt;
+  fx.pop_index = pop_index;
+  fx.hist_ld = ld;
+  fx.pop_hist = pop_out ? f->hist : nullptr;
+  fx.norm_hist = norm_out ? f->hist + (pop_out ? hist : 0) : nullptr;
+  std::vector<int> ids(B);
+  std::iota(ids.begin(), ids.end(), 0);
+  if ((rc = mpc_flowb_tail(c, B, ids, pulses, t0, steps, fx, out))) return rc;
   std::vector<double> h(pop_out || norm_out ? (pop_out ? hist : 0) + (norm_out ? hist : 0) : 0);
   if (!h.empty())
     CK(cudaMemcpyAsync(h.data(), f->hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,

@@ -2,7 +2,9 @@
 // coupling fits on chip (flow_batch.cu).
 #pragma once
 #include <cstddef>
+#include <vector>
 
+#include "batch_types.h"
 #include "ctx.h"
 
 bool mpc_flowb_setup(mpc_ctx* c);   // usable for this system
@@ -24,3 +26,11 @@ int mpc_flowb_propagate(mpc_ctx* c, int B, const mpc_pulse* pulses, const double
                         const double* t_end, double h0, double dt_max, double rtol, double atol,
                         int max_attempts, double* ct, int* accepted, int* rejected,
                         double* t_final);
+
+// The rest of a fixed-step batch that began on the stage GEMM: start states by
+// pulse in the buffer mpc_flowb_states gives ([B][n], device), pulses `ids` with
+// `left` steps from times t (host, by pulse); final states to out [B][n]
+// (device), histories through fx's pointers.
+int mpc_flowb_states(mpc_ctx* c, int B, double2** in);
+int mpc_flowb_tail(mpc_ctx* c, int B, const std::vector<int>& ids, const mpc_pulse* pulses,
+                   const double* t, const int* left, const mpc::FixedStep& fx, double2* out);
