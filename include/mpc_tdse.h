@@ -125,8 +125,9 @@ int mpc_ctx_stream(const mpc_ctx *ctx, void **stream);
 int mpc_rhs(mpc_ctx *ctx, double F, const double *x, double *dxdt);
 
 /* One rkf.do_step(sys, x, t, dt) with the field frozen at F
- * (src/tdse/tdse.cpp:190): 13 stages, 8th-order solution, no
- * renormalisation.  x: host, in/out. */
+ * (src/tdse/tdse.cpp:190): the 8th-order solution, no
+ * renormalisation; formed as the 12 products of the method's stability
+ * polynomial, as the propagation does.  x: host, in/out. */
 int mpc_rk78_step(mpc_ctx *ctx, double F, double dt, double *x);
 
 /* The propagation loop of tdse::propV / tdse::propL

@@ -58,40 +58,58 @@ __global__ void __launch_bounds__(kCombineThreads)
     k_stage_combine(const __grid_constant__ CombineArgs a) {
   const Geometry& g = a.g;
   pdl_trigger();
-  pdl_wait();
   // kCombineLanes consecutive threads share one coefficient: they split its
   // partial sums (strip s and slot s handled by lane s mod kCombineLanes) and
   // reduce them with a fixed shuffle tree; lane 0 finishes the coefficient.
+  // What no launch writes (places, slots, eps, the field) is read before the
+  // wait for the dipole pass.
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = gt / kCombineLanes;
   const int q = gt % kCombineLanes;
   const bool valid = i < g.ntot;
-  int L = 0, r = 0;
-  double2 Q = make_double2(0.0, 0.0), P = make_double2(0.0, 0.0);
+  int L = 0, nq = 0, np = 0;
+  long long qstep = 0;
+  const double2* rp = a.RP;
+  const double2* cp = a.CP;
+  double e = 0.0, F = 0.0;
   if (valid) {
     while (L + 1 < g.nstate_blk && i >= g.state_off[L + 1]) ++L;
-    r = i - g.state_off[L];
+    const int r = i - g.state_off[L];
     if (L < g.nblk) {
       const BlockGeom& b = g.blk[L];
-      const double2* rp = a.RP + b.rp_off + r;
-#pragma unroll 4
-      for (int s = q; s < b.nstrips; s += kCombineLanes) {
-        const double2 v = rp[s * (long long)b.nrow];
-        Q.x = dadd(Q.x, v.x);
-        Q.y = dadd(Q.y, v.y);
-      }
+      rp += b.rp_off + r + q * (long long)b.nrow;
+      qstep = kCombineLanes * (long long)b.nrow;
+      nq = b.nstrips - q;
     }
     if (L > 0) {
-      const BlockGeom& b = g.blk[L - 1];
-      const int gs = b.strip0 + r / kStripW;
-      const int c = r % kStripW;
-      const int s1 = a.strip_slot0[gs + 1];
-      for (int sl = a.strip_slot0[gs] + q; sl < s1; sl += kCombineLanes) {
-        const double2 v = a.CP[(long long)sl * kStripW + c];
-        P.x = dadd(P.x, v.x);
-        P.y = dadd(P.y, v.y);
-      }
+      const int gs = g.blk[L - 1].strip0 + r / kStripW;
+      const int s0 = a.strip_slot0[gs];
+      np = a.strip_slot0[gs + 1] - s0 - q;
+      cp += (s0 + q) * (long long)kStripW + r % kStripW;
     }
+    if (q == 0) {
+      e = a.eps[i];
+      F = a.Ftab[a.step];
+    }
+  }
+  pdl_wait();
+  double2 Q = make_double2(0.0, 0.0), P = make_double2(0.0, 0.0);
+  double2 yi = Q, xi = Q;
+  if (valid && q == 0) {
+    yi = a.y[i];
+    xi = a.x[i];
+  }
+#pragma unroll 4
+  for (; nq > 0; nq -= kCombineLanes, rp += qstep) {
+    const double2 v = *rp;
+    Q.x = dadd(Q.x, v.x);
+    Q.y = dadd(Q.y, v.y);
+  }
+#pragma unroll 4
+  for (; np > 0; np -= kCombineLanes, cp += kCombineLanes * kStripW) {
+    const double2 v = *cp;
+    P.x = dadd(P.x, v.x);
+    P.y = dadd(P.y, v.y);
   }
 #pragma unroll
   for (int o = 1; o < kCombineLanes; o <<= 1) {
@@ -102,12 +120,8 @@ __global__ void __launch_bounds__(kCombineThreads)
   }
   double nsq = 0.0;
   if (valid && q == 0 && a.horner) {
-    const double F = a.Ftab[a.step];
-    const double e = a.eps[i];
     const double vs = a.vscale;
-    const double2 yr = a.y[i];
-    const double2 xi = a.x[i];
-    const double2 y = make_double2(dmul(vs, yr.x), dmul(vs, yr.y));
+    const double2 y = make_double2(dmul(vs, yi.x), dmul(vs, yi.y));
     P = make_double2(dmul(vs, P.x), dmul(vs, P.y));
     Q = make_double2(dmul(vs, Q.x), dmul(vs, Q.y));
     double kre = dmul(e, y.y);
@@ -124,9 +138,7 @@ __global__ void __launch_bounds__(kCombineThreads)
     a.out[i] = o;
     nsq = dadd(dmul(o.x, o.x), dmul(o.y, o.y));
   } else if (valid && q == 0) {
-    const double F = a.Ftab[a.step];
-    const double e = a.eps[i];
-    const double2 y = a.y[i];
+    const double2 y = yi;
     double kre = dmul(e, y.y);
     double kim = dmul(-e, y.x);
     if (a.gauge == 0) {
@@ -146,7 +158,7 @@ __global__ void __launch_bounds__(kCombineThreads)
         const int j = a.coef_j[m];
         kj[m] = (j == a.stage) ? make_double2(kre, kim) : a.k[j * n + i];
       }
-    double2 acc = a.x[i];
+    double2 acc = xi;
 #pragma unroll
     for (int m = 0; m < kNumStages; ++m)
       if (m < a.ncoef) {

@@ -756,7 +756,7 @@ int mpc_rk78_step(mpc_ctx* c, double F, double dt, double* x) {
   CK(cudaMemcpyAsync(c->d_x, x, bytes, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->d_Ftab, &F, sizeof(double), cudaMemcpyHostToDevice, c->stream));
   int rc;
-  if ((rc = rk78_step_dev(c, 0, dt))) return rc;
+  if ((rc = c->stage_form ? rk78_step_dev(c, 0, dt) : horner_step_dev(c, 0, dt))) return rc;
   CK(cudaMemcpyAsync(x, c->d_y, bytes, cudaMemcpyDeviceToHost, c->stream));
   return check_status(c);
 }

@@ -20,11 +20,13 @@ constexpr int kMaxBlocks = 16;      // angular-momentum blocks L = 0..15
 constexpr int kStripW = 256;        // tile width (columns, doubles)
 constexpr int kTileR = 16;          // tile height (rows)
 constexpr int kStages = 4;          // TMA ring depth
+constexpr int kPrefill = 1;         // tiles requested before the previous kernel is done
 constexpr int kConsumerWarps = 8;   // warps that compute; one more issues TMA
 constexpr int kStreamThreads = (kConsumerWarps + 1) * 32;
 constexpr int kTileBytes = kTileR * kStripW * 8;
 constexpr int kYRowBytes = kTileR * 16;          // the tile's stage-vector rows
-constexpr int kRedBytes = kConsumerWarps * kStripW * 16;
+constexpr int kRedWarps = kConsumerWarps / 2;  // column partials staged at a time
+constexpr int kRedBytes = kRedWarps * kStripW * 16;
 constexpr int kRpRows = 512;        // row partials staged per bulk store
 constexpr int kRpStageBytes = 2 * kRpRows * 16;
 constexpr int kStreamSmem =

@@ -16,16 +16,31 @@
 // mbarriers).  Warps 0-7 consume: warp w takes rows 2w and 2w+1
 // of each tile; lane l holds the 8 columns {64j + 2l, 64j + 2l + 1}, j<4, of
 // the current strip.
-//   - Row partials are complete for the strip after a 6-shuffle
-//     reduce-scatter across the warp; they are staged in shared memory (two
-//     buffers of kRpRows rows) and written to RP[strip][row] by one bulk
-//     store per run of consecutive rows.
+//   - Row partials are complete for the strip after a reduce-scatter across
+//     the warp, two tiles at a time where the strip has two (9 shuffles and
+//     one chain of latencies for both, not 12 and two); they are staged in
+//     shared memory (two buffers of kRpRows rows) and written to
+//     RP[strip][row] by one bulk store per run of consecutive rows.
 //   - Column partials accumulate in registers while the CTA walks down a
 //     strip; when the strip (or the CTA's range) ends, the 8 warps' partials
-//     are summed in shared memory (warp order 0..7) and stored as one slot
-//     CP[slot][0..255].
+//     are summed in shared memory (warps 0..3, each with its partner 4..7)
+//     and stored as one slot CP[slot][0..255].
 // Every output is written by exactly one thread in a fixed order, so repeated
 // runs give identical bits.
+//
+// What bounds it: blocks beyond L2 the HBM stream; blocks that fit the tile
+// rate from L2 and, per pass, about 6 us of the combine pass and of latencies
+// at both ends.  The consumers have to stay well ahead of the ring: with one
+// tile at a time (a select per operand for the timed-out case, two shuffle
+// chains) they cost 17-20 % over the bare stream.  Measured, 60 steps on
+// 18,000 states (491 MB of blocks): 63.5 -> 57.7 ms; 150 steps on 5,712
+// states (52 MB): 30.5 -> 25.5 ms.
+// kPrefill: tiles requested while the previous kernel, the combine pass, is
+// still at work.  Their loads queue before the combine's own, whose latency
+// everything waits for: 1 / 2 / 3 / 4 tiles give 25.5 / 25.7 / 26.1 / 26.5 ms
+// on the 52 MB blocks, and no difference beyond the noise on the 491 MB ones.
+// kStages: 3 / 4 / 6 stages give 59.0 / 57.7 / 59.6 ms on the large blocks and
+// 25.6 / 25.7 / 25.9 ms on the small ones, at two tiles of prefill.
 #pragma once
 #include <cuda.h>
 
@@ -81,10 +96,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     const uint64_t stream_policy = make_evict_first_policy();
     const uint64_t keep_policy = make_evict_last_policy();
     const int keep_end = t_begin + (int)(a.keep_frac * (float)(t_end - t_begin));
-    // The dipole blocks do not change between launches: the first ring's
-    // worth of tiles is requested before waiting for the previous kernel;
+    // The dipole blocks do not change between launches: the first kPrefill
+    // tiles are requested before waiting for the previous kernel;
     // their stage-vector rows (written by that kernel) only after it.
-    const int pre = (t_end - t_begin < kStages) ? (t_end - t_begin) : kStages;
+    const int pre = min(t_end - t_begin, kPrefill);
     for (int i = 0; i < pre; ++i) {
       int b, s, rt;
       decode_tile(g, t_begin + i, b, s, rt);
@@ -100,7 +115,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
       int b, s, rt;
       decode_tile(g, t, b, s, rt);
       if (issued >= pre) {
-        if (!mbar_wait_bounded(&empty[stage], (round - 1) & 1, a.status)) break;
+        if (round > 0 && !mbar_wait_bounded(&empty[stage], (round - 1) & 1, a.status)) break;
         mbar_arrive_expect_tx(&full[stage], kTileBytes + kYRowBytes);
         tma_load_2d_hint(tiles + stage * (kTileR * kStripW), &tm.m[b], &full[stage],
                          s * kStripW, rt * kTileR, t < keep_end ? keep_policy : stream_policy);
@@ -130,16 +145,27 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   const int ctid = threadIdx.x;  // 0..255 among consumers
 
   auto flush_cols = [&](int b) {
-    // warp partials -> shared, then a fixed-order sum over warps
+    // warp partials -> shared in two halves (a whole set would cost the ring a
+    // stage), then a fixed-order sum
+    double2* mine = red + (warp % kRedWarps) * kStripW + 2 * lane;
+    if (warp < kRedWarps) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      red[warp * kStripW + 64 * j + 2 * lane] = cacc[2 * j];
-      red[warp * kStripW + 64 * j + 2 * lane + 1] = cacc[2 * j + 1];
+      for (int j = 0; j < 8; ++j) mine[64 * (j / 2) + j % 2] = cacc[j];
+    }
+    named_bar_sync(1, kConsumerWarps * 32);
+    if (warp >= kRedWarps) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        double2 v = mine[64 * (j / 2) + j % 2];
+        v.x += cacc[j].x;
+        v.y += cacc[j].y;
+        mine[64 * (j / 2) + j % 2] = v;
+      }
     }
     named_bar_sync(1, kConsumerWarps * 32);
     double2 acc = red[ctid];
 #pragma unroll
-    for (int w = 1; w < kConsumerWarps; ++w) {
+    for (int w = 1; w < kRedWarps; ++w) {
       const double2 v = red[w * kStripW + ctid];
       acc.x += v.x;
       acc.y += v.y;
@@ -175,19 +201,73 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   // shared memory, so that every consumer warp still reaches each named
   // barrier; the raised status makes the host discard the result.
   bool dead = false;
-  int it = 0;
-  for (int t = t_begin; t < t_end; ++t, ++it) {
-    int b, s, rt;
-    decode_tile(g, t, b, s, rt);
+  int stage = 0, phase = 0;  // of the next tile
+  // The next tile: this warp's two rows' sums over its columns into w (row
+  // 2 warp: re, im; row 2 warp + 1: re, im), its columns' into cacc.
+  auto tile = [&](double* w) {
+    if (!dead && !mbar_wait_bounded(&full[stage], phase, a.status)) dead = true;
+    w[0] = w[1] = w[2] = w[3] = 0.0;
+    if (dead) return;
+    // rows past the block's end meet zero-filled dipole rows, so their
+    // (finite) stage-vector entries contribute nothing
+    const double2 yr0 = yrows[stage * kTileR + 2 * warp];
+    const double2 yr1 = yrows[stage * kTileR + 2 * warp + 1];
+    const double* T = tiles + stage * (kTileR * kStripW);
+    const double* T0 = T + (2 * warp) * kStripW + 2 * lane;
+    const double* T1 = T0 + kStripW;
+    double2 ra = make_double2(0.0, 0.0), rb = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double2 d0 = *reinterpret_cast<const double2*>(T0 + 64 * j);
+      const double2 d1 = *reinterpret_cast<const double2*>(T1 + 64 * j);
+      const double2 c0 = ycol[2 * j], c1 = ycol[2 * j + 1];
+      ra.x = fma(d0.x, c0.x, ra.x); ra.x = fma(d0.y, c1.x, ra.x);
+      ra.y = fma(d0.x, c0.y, ra.y); ra.y = fma(d0.y, c1.y, ra.y);
+      rb.x = fma(d1.x, c0.x, rb.x); rb.x = fma(d1.y, c1.x, rb.x);
+      rb.y = fma(d1.x, c0.y, rb.y); rb.y = fma(d1.y, c1.y, rb.y);
+      double2& q0 = cacc[2 * j];
+      double2& q1 = cacc[2 * j + 1];
+      q0.x = fma(d0.x, yr0.x, q0.x); q0.x = fma(d1.x, yr1.x, q0.x);
+      q0.y = fma(d0.x, yr0.y, q0.y); q0.y = fma(d1.x, yr1.y, q0.y);
+      q1.x = fma(d0.y, yr0.x, q1.x); q1.x = fma(d1.y, yr1.x, q1.x);
+      q1.y = fma(d0.y, yr0.y, q1.y); q1.y = fma(d1.y, yr1.y, q1.y);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[stage]);
+    if (++stage == kStages) {
+      stage = 0;
+      phase ^= 1;
+    }
+    w[0] = ra.x;
+    w[1] = ra.y;
+    w[2] = rb.x;
+    w[3] = rb.y;
+  };
+  // A reduce-scatter step over lane bit OFF: half of the 2 N values stay.
+  auto halve = [&](double* v, int n, int off) {
+    const bool up = (lane & off) != 0;
+    for (int i = 0; i < n; ++i) {
+      const double keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  };
+  int t = t_begin;
+  int b, s, rt;
+  if (t < t_end) decode_tile(g, t, b, s, rt);
+  while (t < t_end) {
     const BlockGeom& bg = g.blk[b];
-    if (b != seg_b || s != seg_s || seg_n == kRpRows || rt * kTileR != seg_r0 + seg_n) {
+    // two tiles of the strip at a time where there are two: their chains and
+    // shuffles overlap, and the eight sums reduce in nine shuffles, not twelve
+    const int two = t + 1 < t_end && rt + 1 < bg.nrtiles ? 1 : 0;
+    if (b != seg_b || s != seg_s || seg_n + kTileR * (1 + two) > kRpRows ||
+        rt * kTileR != seg_r0 + seg_n) {
       flush_rows();
       seg_b = b;
       seg_s = s;
       seg_r0 = rt * kTileR;
     }
-    const int rp_local = rt * kTileR - seg_r0;  // this tile's first row in the buffer
-    seg_n += kTileR;
+    const int rp_local = rt * kTileR - seg_r0;  // the first tile's first row in the buffer
+    seg_n += kTileR * (1 + two);
     if (b != cur_b || s != cur_s) {
       if (cur_b >= 0) flush_cols(cur_b);
       ++slot;
@@ -203,56 +283,38 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         }
       }
     }
-    const int stage = it % kStages;
-    const int round = it / kStages;
-    if (!dead && !mbar_wait_bounded(&full[stage], round & 1, a.status)) dead = true;
-    // rows past the block's end meet zero-filled dipole rows, so their
-    // (finite) stage-vector entries contribute nothing
-    const double2 yr0 = dead ? make_double2(0.0, 0.0) : yrows[stage * kTileR + 2 * warp];
-    const double2 yr1 = dead ? make_double2(0.0, 0.0) : yrows[stage * kTileR + 2 * warp + 1];
-    const double* T = tiles + stage * (kTileR * kStripW);
-    const double* T0 = T + (2 * warp) * kStripW + 2 * lane;
-    const double* T1 = T0 + kStripW;
-    double2 ra = make_double2(0.0, 0.0), rb = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const double2 d0 = dead ? make_double2(0.0, 0.0) : *reinterpret_cast<const double2*>(T0 + 64 * j);
-      const double2 d1 = dead ? make_double2(0.0, 0.0) : *reinterpret_cast<const double2*>(T1 + 64 * j);
-      const double2 c0 = ycol[2 * j], c1 = ycol[2 * j + 1];
-      ra.x = fma(d0.x, c0.x, ra.x); ra.x = fma(d0.y, c1.x, ra.x);
-      ra.y = fma(d0.x, c0.y, ra.y); ra.y = fma(d0.y, c1.y, ra.y);
-      rb.x = fma(d1.x, c0.x, rb.x); rb.x = fma(d1.y, c1.x, rb.x);
-      rb.y = fma(d1.x, c0.y, rb.y); rb.y = fma(d1.y, c1.y, rb.y);
-      double2& q0 = cacc[2 * j];
-      double2& q1 = cacc[2 * j + 1];
-      q0.x = fma(d0.x, yr0.x, q0.x); q0.x = fma(d1.x, yr1.x, q0.x);
-      q0.y = fma(d0.x, yr0.y, q0.y); q0.y = fma(d1.x, yr1.y, q0.y);
-      q1.x = fma(d0.y, yr0.x, q1.x); q1.x = fma(d1.y, yr1.x, q1.x);
-      q1.y = fma(d0.y, yr0.y, q1.y); q1.y = fma(d1.y, yr1.y, q1.y);
+    double w[8];
+    tile(w);
+    double* rp = reinterpret_cast<double*>(rpbuf + rp_cur * kRpRows + rp_local + 2 * warp);
+    if (two) {
+      tile(w + 4);
+      // lane bits 16, 8, 4 -> tile, row, re/im
+      halve(w, 4, 16);
+      halve(w, 2, 8);
+      halve(w, 1, 4);
+      double z = w[0];
+      z += __shfl_xor_sync(0xffffffffu, z, 2);
+      z += __shfl_xor_sync(0xffffffffu, z, 1);
+      if ((lane & 3) == 0)
+        rp[(lane & 16 ? 2 * kTileR : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0)] = z;
+      t += 2;
+      rt += 2;
+    } else {
+      // lane bits 16, 8 -> row, re/im
+      halve(w, 2, 16);
+      halve(w, 1, 8);
+      double z = w[0];
+      z += __shfl_xor_sync(0xffffffffu, z, 4);
+      z += __shfl_xor_sync(0xffffffffu, z, 2);
+      z += __shfl_xor_sync(0xffffffffu, z, 1);
+      if ((lane & 7) == 0) rp[(lane & 16 ? 2 : 0) + (lane & 8 ? 1 : 0)] = z;
+      ++t;
+      ++rt;
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[stage]);
-
-    // reduce-scatter of (ra.x, ra.y, rb.x, rb.y) over the 32 lanes:
-    // lane 0 -> ra.x, lane 8 -> ra.y, lane 16 -> rb.x, lane 24 -> rb.y
-    const bool hi16 = (lane & 16) != 0;
-    const double s0 = hi16 ? ra.x : rb.x, s1 = hi16 ? ra.y : rb.y;
-    const double k0 = hi16 ? rb.x : ra.x, k1 = hi16 ? rb.y : ra.y;
-    const double w0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
-    const double w1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-    const bool hi8 = (lane & 8) != 0;
-    double z = (hi8 ? w1 : w0) + __shfl_xor_sync(0xffffffffu, hi8 ? w0 : w1, 8);
-    z += __shfl_xor_sync(0xffffffffu, z, 4);
-    z += __shfl_xor_sync(0xffffffffu, z, 2);
-    z += __shfl_xor_sync(0xffffffffu, z, 1);
-    if ((lane & 7) == 0) {
-      double* rp = reinterpret_cast<double*>(rpbuf + rp_cur * kRpRows + rp_local + 2 * warp +
-                                             (hi16 ? 1 : 0));
-      rp[hi8 ? 1 : 0] = z;
-    }
+    if (rt >= bg.nrtiles && t < t_end) decode_tile(g, t, b, s, rt);
   }
-  if (cur_b >= 0) flush_cols(cur_b);
   flush_rows();
+  if (cur_b >= 0) flush_cols(cur_b);
   if (ctid == 0) bulk_wait<0>();  // the last stores complete before the grid does
 }
 
