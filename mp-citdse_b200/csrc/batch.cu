@@ -9,6 +9,10 @@
 // matrix, run on the FP64 tensor cores (mma.sync m16n8k8 .f64), with the RK
 // stage epilogue fused into the GEMM's store.
 //
+// Systems whose coupling fits the SMs' registers and shared memory take the
+// persistent batched kernels instead (flow_batch.cu), where those are faster
+// for the number of pulses; a fixed-step batch that narrows moves over.
+//
 // Per attempted step (all active pulses at once):
 //   13 x k_batch_stage   (GEMM + epilogue: k_s, next stage input; the last
 //                         stage also forms x_new, the embedded 7th-order
@@ -16,6 +20,8 @@
 //    1 x k_batch_control (per pulse: accept/reject, next step, stage fields)
 //    1 x k_batch_apply   (accepted pulses: x = x_new / ||x_new||; retired
 //                         pulses write their final state out)
+// A fixed step needs no such pass: its first product normalises, and
+// k_batch_out writes the finished states where the host knows of some.
 // Retired pulses' columns are compacted away so the GEMM narrows.
 // Step control and error norm are those of the CPU oracle's adaptive driver:
 //   err = max_i |e_i| / (atol + rtol*max(|x_i|, |x_new_i|)),
@@ -503,6 +509,7 @@ StageArgs stage_args(mpc_ctx* c, int s, int ncol, double rtol, double atol, bool
   a.fs_stride = b->ldc;
   a.ws = b->ws;
   a.cnt = b->cnt;
+  a.status = c->d_status;
   a.nrm = b->c.nrm;
   a.Xw = b->X;
   a.g = c->g;
@@ -933,7 +940,7 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
   CK(cudaGetLastError());
   ca.mode = 1;
   // pulses with nothing to do are retired by the start: write their states
-  // out (the control kernel itself does in fixed-step mode)
+  // out (k_batch_out below does in fixed-step mode)
   if (!fx.on) {
     aa.ncol = ncol;
     k_batch_apply<<<blocks_for((long long)n * ncol, 256), 256, 0, c->stream>>>(aa);

@@ -265,6 +265,7 @@ StageArgs fb_args(mpc_ctx* c, int stage, int step) {
   s.fpart = a->fpart;
   s.ws = a->ws;
   s.cnt = a->cnt;
+  s.status = c->d_status;
   s.g = c->g;
   return s;
 }

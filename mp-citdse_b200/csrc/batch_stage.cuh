@@ -58,6 +58,17 @@ template <int BN_, int NST_, int SPLIT_> constexpr int stage_smem() {
   return paired<BN_, SPLIT_>() ? pair_slots<NST_>() * 2 * (A_STAGE + b_stage<BN_>()) * 8
                                : batch_smem<BN_, NST_>();
 }
+// The persistent launch's wider tiles run one chunk at a time on a ring with
+// barriers per slot (Ring, below) in place of one CTA barrier per chunk or pair:
+// fixed steps of 64 pulses on 11,914 states 6.13 -> 5.44 ms (64 columns) and
+// 6.33 -> 5.75 ms (32), of 256 pulses on 1752 states 598 -> 552 us (32; 64: 765
+// -> 751).  Narrower tiles and the launches per product gain nothing (16 columns
+// +2 %; per product -10 to +2 %, where the persistent launch is the faster) and
+// keep the pairs and the CTA barrier.
+template <int BN_> constexpr bool ringed() { return BN_ >= 32; }
+template <int BN_, int NST_> constexpr int horner_smem() {
+  return ringed<BN_>() ? batch_smem<BN_, NST_>() : stage_smem<BN_, NST_, 0>();
+}
 
 __constant__ double c_A[13][13];
 __constant__ double c_B8[13];
@@ -127,6 +138,7 @@ struct StageArgs {
   // to finish adds the first one's partial (workspace) and runs the epilogue
   double* ws;            // [row tiles x column tiles][2][BM x BN]
   int* cnt;              // [row tiles x column tiles] arrivals (left at zero)
+  unsigned* status;
   Geometry g;
 };
 
@@ -291,9 +303,61 @@ __device__ __forceinline__ void pair_mma(const double* AsP, const double* BsP, c
     pair_mma_body<BN, false>(AsP, BsP, AsQ, BsQ, wm, wn, gq, tq, nksP, nksQ, mt_lim, accP, accQ);
 }
 
-template <int BN, int NSTB, int MODE, int SPLIT>
+// The ring's barriers and this thread's place in it, kept from tile to tile.
+// full[i]: every thread's copies into slot i have landed; empty[i]: every warp
+// has read it.  With a CTA barrier per chunk warps spent a quarter of their time
+// there; here one can run a chunk ahead of another.  The next load is issued
+// after a chunk's products, so that the slot it goes to, the one before, is long
+// free (after the first or second of a chunk's four k-steps: spills, +10 %).
+struct Ring {
+  uint64_t* full;
+  uint64_t* empty;
+  int slot = 0, phase = 0;       // of the next chunk (or pair) to read
+  int lslot = 0, lphase = 1;     // of the next one to load
+  bool dead = false;             // a wait ran out: no more waiting, the call fails
+  __device__ Ring(uint64_t* b, int n) : full(b), empty(b + n) {
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < n; ++i) {
+        mbar_init(full + i, BTHREADS);
+        mbar_init(empty + i, BTHREADS / 32);
+      }
+      fence_mbar_init();
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ void wait_full(unsigned* status) {
+    if (!dead && !mbar_wait_bounded(full + slot, phase, status)) dead = true;
+    __syncwarp();
+  }
+  template <int N>
+  __device__ __forceinline__ void release() {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(empty + slot);
+    if (++slot == N) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+  // (a fresh barrier's preceding phase counts as complete: the first round
+  // of loads does not wait)
+  __device__ __forceinline__ void wait_empty(unsigned* status) {
+    if (!dead && !mbar_wait_bounded(empty + lslot, lphase, status)) dead = true;
+  }
+  template <int N>
+  __device__ __forceinline__ void loaded() {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(full + lslot))
+                 : "memory");
+    if (++lslot == N) {
+      lslot = 0;
+      lphase ^= 1;
+    }
+  }
+};
+constexpr int kMaxSlots = 6;
+
+template <int BN, int NSTB, int MODE, int SPLIT, bool RING>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, const ProdSel& ps, const int bid,
-                                           double* bsm) {
+                                           double* bsm, Ring* ring) {
   constexpr int WGM = Tile<BN>::WGM, WMT = Tile<BN>::WMT, WNT = Tile<BN>::WNT;
   constexpr int LDB = BN + 4;
   constexpr int B_STAGE = b_stage<BN>();
@@ -404,7 +468,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const ProdSel& ps
 #pragma unroll
       for (int v = 0; v < 4; ++v) accP[i][j][v] = accQ[i][j][v] = 0.0;
 
-  if constexpr (paired<BN, SPLIT>()) {
+  if constexpr (paired<BN, SPLIT>() && !RING) {
     // slot i holds P chunk i (first half) and Q chunk i (second half)
     constexpr int NSP = pair_slots<NSTB>();
     constexpr int CH = A_STAGE + B_STAGE;
@@ -438,21 +502,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const ProdSel& ps
     const int ch0 = (SPLIT && zk == 1) ? nchP : 0;
     const int ch1 = (SPLIT && zk == 0) ? nchP : nch;
     const int nmine = ch1 - ch0;
-    for (int p = 0; p < NSTB - 1; ++p) {
-      if (p < nmine) load_chunk(ch0 + p, bsm + p * (A_STAGE + B_STAGE));
-      cp_commit();
-    }
     // this CTA's P chunks come first (local indices [0, nPm)), then its Q chunks
     const int nPm = (SPLIT && zk == 1) ? 0 : nchP;
-    for (int ci = 0; ci < nmine; ++ci) {
-      cp_wait<NSTB - 2>();
-      __syncthreads();
-      {
-        const int nx = ci + NSTB - 1;
-        if (nx < nmine) load_chunk(ch0 + nx, bsm + (nx % NSTB) * (A_STAGE + B_STAGE));
-        cp_commit();
-      }
-      const double* As = bsm + (ci % NSTB) * (A_STAGE + B_STAGE);
+    auto mma = [&](int ci, int slot) {
+      const double* As = bsm + slot * (A_STAGE + B_STAGE);
       const double* Bs = As + A_STAGE;
       // valid k-steps of this chunk: the coupled block's columns left from k0
       const int chg = ch0 + ci;
@@ -462,8 +515,36 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const ProdSel& ps
         chunk_mma<BN, true>(As, Bs, wm, wn, gq, tq, nks, mt_lim, accP);
       else
         chunk_mma<BN, false>(As, Bs, wm, wn, gq, tq, nks, mt_lim, accQ);
+    };
+    if constexpr (RING) {
+      auto load_next = [&](int ci) {
+        if (ci >= nmine) return;
+        ring->wait_empty(a.status);
+        load_chunk(ch0 + ci, bsm + ring->lslot * (A_STAGE + B_STAGE));
+        ring->loaded<NSTB>();
+      };
+      for (int p = 0; p < NSTB - 1; ++p) load_next(p);
+      for (int ci = 0; ci < nmine; ++ci) {
+        ring->wait_full(a.status);
+        mma(ci, ring->slot);
+        ring->release<NSTB>();
+        load_next(ci + NSTB - 1);
+      }
+    } else {
+      for (int p = 0; p < NSTB - 1; ++p) {
+        if (p < nmine) load_chunk(ch0 + p, bsm + p * (A_STAGE + B_STAGE));
+        cp_commit();
+      }
+      for (int ci = 0; ci < nmine; ++ci) {
+        cp_wait<NSTB - 2>();
+        __syncthreads();
+        const int nx = ci + NSTB - 1;
+        if (nx < nmine) load_chunk(ch0 + nx, bsm + (nx % NSTB) * (A_STAGE + B_STAGE));
+        cp_commit();
+        mma(ci, ci % NSTB);
+      }
+      cp_wait<0>();
     }
-    cp_wait<0>();
   }
   if constexpr (SPLIT) {
     // publish this half, then the tile's second arrival takes over
@@ -824,7 +905,7 @@ template <int BN, int NSTB, int MODE, int SPLIT>
 __global__ void __launch_bounds__(BTHREADS, 2) k_batch_stage(const __grid_constant__ StageArgs a) {
   extern __shared__ __align__(16) double bsm[];
   pdl_trigger();
-  stage_tile<BN, NSTB, MODE, SPLIT>(a, prod_sel(a), (int)blockIdx.x, bsm);
+  stage_tile<BN, NSTB, MODE, SPLIT, false>(a, prod_sel(a), (int)blockIdx.x, bsm, nullptr);
 }
 
 // The 12 Horner products of one fixed step in one persistent launch.  Work
@@ -858,6 +939,8 @@ template <int BN, int NSTB>
 __global__ void __launch_bounds__(BTHREADS, 2) k_batch_horner(const __grid_constant__ HornerArgs h) {
   extern __shared__ __align__(16) double bsm[];
   __shared__ int s_item, s_dead;
+  __shared__ uint64_t bars[2 * kMaxSlots];
+  Ring ring(bars, NSTB);
   const Geometry& g = h.a.g;
   const int nrt = h.a.nrowtiles, ncolt = h.ncolt;
   const int per = nrt * ncolt, total = 12 * per;
@@ -914,7 +997,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) k_batch_horner(const __grid_const
     ps.hg = c_G[11 - p];
     ps.vscale = (p == 0) ? c_G[12] : 1.0;
     ps.hlast = (p == 11) ? 1 : 0;
-    stage_tile<BN, NSTB, 2, 0>(h.a, ps, rtile * ncolt + ct, bsm);
+    stage_tile<BN, NSTB, 2, 0, ringed<BN>()>(h.a, ps, rtile * ncolt + ct, bsm, &ring);
     __syncthreads();   // every thread's stores of the tile are issued
     if (threadIdx.x == 0) {
       __threadfence();
@@ -953,7 +1036,7 @@ inline int default_variant(int ncol, int nrt) {
 }
 // ... and of a whole fixed step: at 188 and 208 tiles (between one and one and
 // a half per SM) and from 960 the persistent launch was faster (1.49 against
-// 1.9 ms at 11,914 states and 4 pulses, 6.17 against 6.6 at 64).
+// 1.9 ms at 11,914 states and 4 pulses, 5.44 against 6.3 at 64).
 inline bool default_persistent(int ncol, int nrt) {
   const int T = tiles16(ncol, nrt);
   return (T > 150 && T <= 222) || T > 900;
@@ -990,7 +1073,7 @@ cudaError_t launch_horner_tile(cudaStream_t st, const HornerArgs& h, int sms, in
   static int per_sm = 0;   // resident CTAs per SM (the same on every B200)
   if (per_sm == 0) {
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, k_batch_horner<BN, NST>, BTHREADS, stage_smem<BN, NST, 0>());
+        &per_sm, k_batch_horner<BN, NST>, BTHREADS, horner_smem<BN, NST>());
     if (e != cudaSuccess) {
       per_sm = 0;
       return e;
@@ -998,7 +1081,7 @@ cudaError_t launch_horner_tile(cudaStream_t st, const HornerArgs& h, int sms, in
   }
   const int grid = std::max(1, std::min(items, std::max(per_sm, 1) * sms));
   // plain stream order: the counters' clear right before must be complete
-  k_batch_horner<BN, NST><<<grid, BTHREADS, stage_smem<BN, NST, 0>(), st>>>(h);
+  k_batch_horner<BN, NST><<<grid, BTHREADS, horner_smem<BN, NST>(), st>>>(h);
   return cudaGetLastError();
 }
 
@@ -1051,7 +1134,7 @@ cudaError_t set_stage_attrs() {
 #define MPC_HORNER_ATTR(BN, NST)                                                          \
   if ((e = cudaFuncSetAttribute(k_batch_horner<BN, NST>,                                  \
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,             \
-                                stage_smem<BN, NST, 0>())) != cudaSuccess)               \
+                                horner_smem<BN, NST>())) != cudaSuccess)               \
     return e;
     MPC_HORNER_ATTR(16, 3)
     MPC_HORNER_ATTR(16, 6)
