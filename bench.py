@@ -323,11 +323,11 @@ def measure_batched_ref(local, stream_cls, rank=0, world=1, dist=None, dt=0.05):
     # warm-up at full width (graph capture per width, module loads)
     ctx.batch_advance(pulses, 0.0, dt, [40] * B, X0)
     ctx.sync()
-    plan = ctx.batch_fixed_plan()
     e0.record(st)
     X = ctx.batch_advance(pulses, 0.0, dt, steps, X0)
     e1.record(st)
     ctx.sync()
+    plan = ctx.batch_fixed_plan()
     sec = e0.elapsed_time(e1) / 1000.0
     done = float(sum(steps))
     # every pulse active: the first 400 steps of all of them in one call
@@ -929,13 +929,13 @@ def main():
         bytes_per_launch = 8 * S + 16 * ntot
         avg_s = rhs_ms / rhs_n / 1000.0
     else:
-        # resident path: one launch runs every step; its coupling rows stay in
-        # shared memory, so the figure is the dipole bytes a pass would stream
-        # per right-hand side, over the time of one right-hand side
-        kernel = "k_prop_resident"
+        # resident path: one launch runs every step; its coupling rows stay on
+        # chip, so the figure is the dipole bytes a pass would stream per
+        # product, over the time of one of a step's 12 products
+        kernel = "k_flow_forward"
         bytes_per_launch = 8 * S + 16 * ntot
-        avg_s = res_ms / 1000.0 / (13 * prof_steps)
-        rhs_ms, rhs_n = res_ms, 13 * prof_steps
+        avg_s = res_ms / 1000.0 / (12 * prof_steps)
+        rhs_ms, rhs_n = res_ms, 12 * prof_steps
     achieved = bytes_per_launch / avg_s / 1e9
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "rhs_stream_traffic.json")

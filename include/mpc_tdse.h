@@ -83,12 +83,12 @@ int mpc_ctx_create(int L_max, const int *state_sz, const double *eig, const doub
 int mpc_ctx_destroy(mpc_ctx *ctx);
 
 /* Which kernels run mpc_propagate / mpc_advance:
- *   MPC_PATH_AUTO (0)      resident when the coupling fits in shared memory,
+ *   MPC_PATH_AUTO (0)      resident when the coupling fits on chip,
  *                          streaming otherwise (default);
  *   MPC_PATH_STREAMING (1) per-stage kernels streaming the dipole blocks
  *                          from HBM (any size);
  *   MPC_PATH_RESIDENT (2)  one persistent cooperative kernel per call, each
- *                          CTA holding its rows' coupling in shared memory
+ *                          CTA holding its rows' coupling on chip
  *                          (MPC_ERR_ARG if the system does not fit).
  * Both give the same results within rounding (tested). */
 #define MPC_PATH_AUTO 0
@@ -99,16 +99,16 @@ int mpc_ctx_get_path(mpc_ctx *ctx);   /* the path mpc_advance will take */
 
 /* Failure detection (new: the reference has no device code to watch).  The
  * persistent cooperative kernels (the resident single-pulse propagation, its
- * adjoint sweep and the resident batched tail) meet at grid barriers whose
- * waits are bounded: a CTA that waits longer than this limit (default 2 s)
- * stops, every other CTA stops at its own bounded wait, the call returns
+ * adjoint sweep, and their batched forms) wait for each other's rows, counts
+ * or grid barriers, all bounded: a CTA that waits longer than this limit
+ * (default 2 s) stops, every other CTA stops at its own bounded wait, the call returns
  * MPC_ERR_DEVICE ("wait timeout") and the context stays usable.  seconds in
  * [1e-6, 60].  The streaming kernel's TMA ring waits keep a fixed 2 s bound. */
 int mpc_ctx_set_wait_limit(mpc_ctx *ctx, double seconds);
 
 /* Fault injection for tests of the failure detection above: the next
- * persistent launch on this context gets grid-barrier targets one arrival
- * beyond what its CTAs can make, so its first barrier wait runs out after the
+ * persistent launch on this context gets arrival targets one beyond what its
+ * CTAs can make, so its first such wait runs out after the
  * wait limit and the call reports the timeout.  Later launches are normal. */
 int mpc_ctx_inject_barrier_timeout(mpc_ctx *ctx);
 
@@ -189,8 +189,9 @@ int mpc_batch_propagate(mpc_ctx *ctx, int B, const mpc_pulse *pulses, const doub
  * F_b(t_b + dt) is frozen for the 13 stages, one RKF78 step (8th-order
  * solution), t_b += dt, c_b /= ||c_b||.  Pulse b runs steps[b] steps from
  * t0[b]; a pulse that has finished retires and the batch narrows (each stage
- * is one FP64 tensor-core GEMM over the active pulses; the last few pulses
- * finish in the persistent resident kernel when the coupling fits on chip).
+ * is one FP64 tensor-core GEMM over the active pulses; when the coupling fits
+ * on chip, batches that are narrow or have become so run in one persistent
+ * launch with the coupling resident).
  * ct: host [B][2*size] in/out.  Optional host outputs (NULL to skip), with
  * M = max(steps):
  *   pop_out [B][M+1]   |c_b[pop_index]|^2 at t0[b] and after every step

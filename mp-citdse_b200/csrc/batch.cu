@@ -536,10 +536,9 @@ int horner_plan(mpc_ctx* c, int ncol) {
     return kPlanPerProduct + c->forced_variant;
   const int j = width_bucket(ncol);
   if (j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned) return b->hplan[j];
-  const int v = default_variant(ncol, b->nrowtiles);
-  return default_persistent(ncol, b->nrowtiles) ? v : kPlanPerProduct + v;
+  const int v = default_persistent(ncol, b->nrowtiles);
+  return v >= 0 ? v : kPlanPerProduct + default_variant(ncol, b->nrowtiles);
 }
-
 
 int launch_horner_persistent_v(mpc_ctx* c, int ncol, int v) {
   mpc_batch_state* b = c->batch;

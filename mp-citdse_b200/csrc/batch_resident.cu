@@ -4,7 +4,8 @@
 //
 // When a batch has narrowed to at most 8 pulses, the streamed GEMM path
 // (batch.cu) is bound by per-launch latency rather than by work.  This kernel
-// takes over instead.  Each of G CTAs (one per SM) owns a contiguous range of
+// takes over instead, for the systems that the persistent batched kernels
+// (flow_batch.cu) have no layout for and that fit shared memory all the same.  Each of G CTAs (one per SM) owns a contiguous range of
 // rows of one state block L and keeps their coupling rows in shared memory
 // for the whole run (column r of D_{L-1} and row r of D_L, the latter
 // negated in the velocity gauge), as the single-pulse resident kernel does.

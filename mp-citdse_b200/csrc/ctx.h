@@ -95,10 +95,9 @@ struct mpc_ctx {
   // width (tests of that path; it is correct at any width, not always faster)
   bool force_persist = false;
   // MPC_FORCE_TMA=s at context creation: the batched fixed step as the
-  // TMA-fed product launches on TMA tile shape s - 1 at every width (tests);
-  // MPC_NO_TMA=1: the fixed-step tuner leaves the TMA-fed launches out
+  // TMA-fed product launches on TMA tile shape s - 1 at every width (tests;
+  // no plan picks them: see batch.cu)
   int force_tma = 0;
-  bool no_tma = false;
   // MPC_STAGE_FORM=1 at context creation: the streamed single-pulse steps as
   // 13 stages instead of the 12 Horner products of the stability polynomial
   bool stage_form = false;

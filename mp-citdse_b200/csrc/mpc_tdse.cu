@@ -581,7 +581,6 @@ int mpc_ctx_create(int L_max, const int* state_sz, const double* eig, const doub
   c->no_persist = std::getenv("MPC_NO_PERSIST") != nullptr;
   c->force_persist = std::getenv("MPC_FORCE_PERSIST") != nullptr;
   if (const char* ft = std::getenv("MPC_FORCE_TMA")) c->force_tma = std::max(0, std::atoi(ft));
-  c->no_tma = std::getenv("MPC_NO_TMA") != nullptr;
   c->stage_form = std::getenv("MPC_STAGE_FORM") != nullptr;
   c->gauge = gauge;
   c->n.assign(state_sz, state_sz + L_max + 1);
