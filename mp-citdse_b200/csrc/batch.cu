@@ -536,7 +536,7 @@ int horner_plan(mpc_ctx* c, int ncol) {
     return kPlanPerProduct + c->forced_variant;
   const int j = width_bucket(ncol);
   if (j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned) return b->hplan[j];
-  const int v = default_persistent(ncol, b->nrowtiles);
+  const int v = default_persistent(ncol, b->nrowtiles, c->g.nstate_blk);
   return v >= 0 ? v : kPlanPerProduct + default_variant(ncol, b->nrowtiles);
 }
 

@@ -1027,23 +1027,26 @@ inline int width_bucket(int ncol) {
 // Before tuning: by the number T of 64 x 16 tiles, on 148 SMs with two CTAs
 // each.  The tuner's picks for 12 Horner products on 1752 to 13,200 states (30 to
 // 208 row tiles) and 1 to 256 pulses: the split (twice the CTAs) up to T = 63;
-// whole tiles with the deep ring, a CTA per SM, at 118 to 208; the shallow ring
+// whole tiles with the deep ring, a CTA per SM, at 118 to 228; the shallow ring
 // (two CTAs per SM) from 236 to 832; wider tiles from 960, 64 columns from 1504.
 inline int tiles16(int ncol, int nrt) { return nrt * ((2 * ncol + 15) / 16); }
 inline int default_variant(int ncol, int nrt) {
   const int T = tiles16(ncol, nrt);
-  return T <= 100 ? 5 : T <= 222 ? 1 : T <= 900 ? 0 : T <= 1300 ? 2 : 4;
+  return T <= 100 ? 5 : T <= 232 ? 1 : T <= 900 ? 0 : T <= 1300 ? 2 : 4;
 }
 // ... and of a whole fixed step: the variant of the persistent launch, or -1 for
 // one launch per product, where the latter was the faster.  One wave and a half of
-// deep-ring CTAs (T = 162 to 208: 690 against 768 us at 5,071 states and 16
-// pulses, 1.61 against 1.64 ms at 11,382 and 6), then 32 columns (T = 720 to
+// deep-ring CTAs where the tiles are deep enough to hide the hand-over (T = 162 to
+// 208: 690 against 768 us at 5,071 states in 4 blocks and 16 pulses, 1.54
+// against 1.72 ms at 11,914 in 5 and 6; but 480 against 390 us at 3,505 in 5
+// and 20: the line is drawn at 1000 states per block), then 32 columns (T = 720 to
 // 1448: 3.55 against 3.86 ms at 11,382 states and 32 pulses, 1.73 against 1.97
 // at 5,800 and 64; at 540 3.56 against 3.25), then 64 columns (T = 1504: 5.44
 // against 5.65 ms with 32 and 6.3 per product, at 11,914 states and 64 pulses).
-inline int default_persistent(int ncol, int nrt) {
+inline int default_persistent(int ncol, int nrt, int nblocks) {
   const int T = tiles16(ncol, nrt);
-  return T <= 150 ? -1 : T <= 222 ? 1 : T <= 640 ? -1 : T <= 1470 ? 2 : 4;
+  if (T > 150 && T <= 232) return nrt * BM >= 1000 * nblocks ? 1 : -1;
+  return T <= 640 ? -1 : T <= 1470 ? 2 : 4;
 }
 
 template <int BN, int NST, int MODE, int SPLIT>
