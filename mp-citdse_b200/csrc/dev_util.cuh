@@ -95,6 +95,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same until %globaltimer passes `deadline`, raising nothing.
+__device__ __forceinline__ bool mbar_wait_until(uint64_t* bar, uint32_t parity,
+                                                unsigned long long deadline) {
+  while (!mbar_try_wait(bar, parity))
+    if (globaltimer_ns() > deadline) return mbar_try_wait(bar, parity);
+  return true;
+}
+
 // 2-D tiled TMA load global -> shared, completing on `bar` (tx bytes).
 // The x coordinate (innermost, in elements) must be a multiple of 2 for
 // 8-byte elements: callers pass multiples of the 256-column strip width.

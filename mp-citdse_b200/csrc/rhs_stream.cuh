@@ -103,19 +103,23 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     for (int i = 0; i < pre; ++i) {
       int b, s, rt;
       decode_tile(g, t_begin + i, b, s, rt);
-      mbar_arrive_expect_tx(&full[i], kTileBytes + kYRowBytes);
+      mbar_arrive_expect_tx(&full[i], kTileBytes + kYRowBytes + (i == 0 ? a.tx_skew : 0u));
       tma_load_2d_hint(tiles + i * (kTileR * kStripW), &tm.m[b], &full[i], s * kStripW,
                        rt * kTileR, t_begin + i < keep_end ? keep_policy : stream_policy);
     }
     pdl_wait();
     int issued = 0;
+    bool late = false;   // the consumers gave up
     for (int t = t_begin; t < t_end; ++t, ++issued) {
       const int stage = issued % kStages;
       const int round = issued / kStages;
       int b, s, rt;
       decode_tile(g, t, b, s, rt);
       if (issued >= pre) {
-        if (round > 0 && !mbar_wait_bounded(&empty[stage], (round - 1) & 1, a.status)) break;
+        if (round > 0 && !mbar_wait_bounded(&empty[stage], (round - 1) & 1, a.status)) {
+          late = true;
+          break;
+        }
         mbar_arrive_expect_tx(&full[stage], kTileBytes + kYRowBytes);
         tma_load_2d_hint(tiles + stage * (kTileR * kStripW), &tm.m[b], &full[stage],
                          s * kStripW, rt * kTileR, t < keep_end ? keep_policy : stream_policy);
@@ -126,12 +130,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
                 &full[stage]);
     }
     // Do not leave while a load is in flight: wait until every issued tile
-    // was released by the consumers, or, if they gave up, until it landed.
+    // was released by the consumers, or, once they gave up, until it landed,
+    // with one limit for all that is left.
+    unsigned long long deadline = late ? globaltimer_ns() + kWaitLimitNs : 0;
     for (int i = (issued > kStages ? issued - kStages : 0); i < issued; ++i) {
       const int stage = i % kStages;
       const int round = i / kStages;
-      if (!mbar_wait_bounded(&empty[stage], round & 1, a.status))
-        mbar_wait_bounded(&full[stage], round & 1, a.status);
+      if (!late && !mbar_wait_bounded(&empty[stage], round & 1, a.status)) {
+        late = true;
+        deadline = globaltimer_ns() + kWaitLimitNs;
+      }
+      if (late) mbar_wait_until(&full[stage], round & 1, deadline);
     }
     return;
   }
@@ -199,13 +208,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
 
   // After a timed-out wait the warp keeps walking its tiles without reading
   // shared memory, so that every consumer warp still reaches each named
-  // barrier; the raised status makes the host discard the result.
+  // barrier; the raised status makes the host discard the result.  The warp
+  // decides as one (a lane's wait may run out where another's comes through),
+  // since the lanes meet again in the reductions.  It releases no more slots:
+  // the producer stops at its next wait for one.
   bool dead = false;
   int stage = 0, phase = 0;  // of the next tile
   // The next tile: this warp's two rows' sums over its columns into w (row
   // 2 warp: re, im; row 2 warp + 1: re, im), its columns' into cacc.
   auto tile = [&](double* w) {
-    if (!dead && !mbar_wait_bounded(&full[stage], phase, a.status)) dead = true;
+    if (!dead)
+      dead = __any_sync(0xffffffffu, !mbar_wait_bounded(&full[stage], phase, a.status));
     w[0] = w[1] = w[2] = w[3] = 0.0;
     if (dead) return;
     // rows past the block's end meet zero-filled dipole rows, so their

@@ -21,6 +21,9 @@ struct StreamArgs {
   // the first keep_frac of every CTA's tiles are loaded with an L2 evict-last
   // hint (they stay in L2 from pass to pass), the rest evict-first
   float keep_frac;
+  // 0; else bytes more than its load brings that each CTA's first tile waits for
+  // (a test's wait that runs out)
+  unsigned tx_skew;
   Geometry g;
 };
 

@@ -465,8 +465,9 @@ class Context:
         _check(lib().mpc_ctx_set_wait_limit(self._h, float(seconds)))
 
     def inject_barrier_timeout(self):
-        """Test hook: the next persistent launch gets a grid barrier that
-        cannot complete, so its bounded wait runs out."""
+        """Test hook: the next persistent launch (or dipole-streaming launch, if
+        that comes first) gets a wait that cannot complete, so its limit runs
+        out."""
         _check(lib().mpc_ctx_inject_barrier_timeout(self._h))
 
     def profile(self, on=True):

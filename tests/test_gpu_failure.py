@@ -132,6 +132,31 @@ def test_persistent_batched_step_dependency_timeout_is_reported(monkeypatch):
     assert np.array_equal(Xa, Xb)
 
 
+@pytest.mark.parametrize("n", [[60, 70, 50], [1300, 1401, 1207]], ids=["short", "long"])
+def test_streamed_ring_timeout_is_reported_and_bounded(n):
+    """The dipole-streaming kernel with a first tile that never counts as there:
+    the consumers' waits run out after 2 s, the producer's at about the same
+    time, and what is left of the loads has one more limit, so the call reports
+    the timeout within 4 s and a little -- with fewer tiles per CTA than the ring
+    has slots (the producer has nothing left to issue) and with more -- and the
+    same context then gives the bits it gave before."""
+    import time
+
+    s = random_system(n, gauge="l", seed=3, e_max=8.0)
+    x = np.random.default_rng(1).standard_normal(s.ntot).astype(complex)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.set_path("streaming")
+        want = ctx.rhs(0.3, x)
+        ctx.inject_barrier_timeout()
+        t = time.perf_counter()
+        with pytest.raises(mpc_tdse.MpcError) as ei:
+            ctx.rhs(0.3, x)
+        t = time.perf_counter() - t
+        assert ei.value.code == -3 and "wait timeout" in str(ei.value)
+        assert 1.9 < t < 5.0
+        assert np.array_equal(ctx.rhs(0.3, x), want)
+
+
 @pytest.mark.parametrize("path", ["streaming", "resident"])
 def test_nan_in_host_state_raises_nonfinite_status(path):
     s = random_system([40, 57, 33], gauge="v", seed=11, e_max=4.0)
