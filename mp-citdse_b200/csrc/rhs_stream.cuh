@@ -206,21 +206,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     seg_n = 0;
   };
 
-  // After a timed-out wait the warp keeps walking its tiles without reading
-  // shared memory, so that every consumer warp still reaches each named
-  // barrier; the raised status makes the host discard the result.  The warp
-  // decides as one (a lane's wait may run out where another's comes through),
-  // since the lanes meet again in the reductions.  It releases no more slots:
-  // the producer stops at its next wait for one.
+  // After a timed-out wait a lane keeps walking its tiles, on whatever the slots
+  // hold, so that its warp stays together in the reductions (another lane's wait
+  // may have come through) and reaches each named barrier; the raised status
+  // makes the host discard the result.  Slots are released by lane 0, as long as
+  // its own waits come through: the producer stops at its next wait for one.
+  // (The warp's vote on each wait instead: +0.4 % on 52 MB of blocks.)
   bool dead = false;
   int stage = 0, phase = 0;  // of the next tile
   // The next tile: this warp's two rows' sums over its columns into w (row
   // 2 warp: re, im; row 2 warp + 1: re, im), its columns' into cacc.
   auto tile = [&](double* w) {
-    if (!dead)
-      dead = __any_sync(0xffffffffu, !mbar_wait_bounded(&full[stage], phase, a.status));
-    w[0] = w[1] = w[2] = w[3] = 0.0;
-    if (dead) return;
+    if (!dead && !mbar_wait_bounded(&full[stage], phase, a.status)) dead = true;
     // rows past the block's end meet zero-filled dipole rows, so their
     // (finite) stage-vector entries contribute nothing
     const double2 yr0 = yrows[stage * kTileR + 2 * warp];
@@ -246,7 +243,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
       q1.y = fma(d0.y, yr0.y, q1.y); q1.y = fma(d1.y, yr1.y, q1.y);
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[stage]);
+    if (lane == 0 && !dead) mbar_arrive(&empty[stage]);
     if (++stage == kStages) {
       stage = 0;
       phase ^= 1;
