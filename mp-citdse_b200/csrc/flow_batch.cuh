@@ -287,11 +287,21 @@ __device__ __forceinline__ double2 fb_m(int gauge, double e, double F, double2 v
 }
 
 // Waits until the helper is done with chunk c up to `step`; false if the
-// helper gave up (its own waits are bounded).
+// helper gave up (its own waits are bounded).  What the helper wrote before its
+// word is plain shared memory: the fence orders the reads after the spin.
 __device__ __forceinline__ bool fb_await(FbCtl& ctl, int c, int step) {
-  while (ctl.step[c] < step)
-    if (ctl.hdead || ctl.mexit) return ctl.step[c] >= step;
-  return true;
+  bool ok = true;
+  while (ok && ctl.step[c] < step)
+    if (ctl.hdead || ctl.mexit) ok = ctl.step[c] >= step;
+  __threadfence_block();
+  return ok;
+}
+
+// The compute warps have finished one more (step, chunk) pair, said by their
+// thread 0 after the CTA's barrier.
+__device__ __forceinline__ void fb_tell(FbCtl& ctl) {
+  __threadfence_block();
+  ctl.progress = ctl.progress + 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -436,7 +446,7 @@ __device__ void fb_fixed_main(const FbArgs& a, FbCtl& ctl, const FbView& u, doub
                         canonical(t));
           }
           __syncwarp();
-          if (tid == 0) ctl.progress = ctl.progress + 1;
+          if (tid == 0) fb_tell(ctl);
         }
       }
     }
@@ -467,10 +477,11 @@ __device__ __forceinline__ bool fb_count(const unsigned long long* ctr, unsigned
 __device__ __forceinline__ void fb_arrive(unsigned long long* ctr) {
   asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(1ull) : "memory");
 }
-// Waits for the compute warps' `events`-th (step, chunk) pair.
+// Waits, in the helper, for the compute warps' `events`-th (step, chunk) pair.
 __device__ __forceinline__ bool fb_progress(FbCtl& ctl, int events) {
   bool ok = true;
   while (ok && ctl.progress < events) ok = ctl.mexit == 0 || ctl.progress >= events;
+  __threadfence_block();
   return __all_sync(0xffffffffu, ok);
 }
 
@@ -686,7 +697,7 @@ __device__ void fb_adj_main(const FbArgs& a, FbCtl& ctl, const FbView& u, double
             for (int k = 1; k < FW; ++k) t += red8[k][tid];
             a.fpart[(((long long)n * a.nch + c * a.ng + u.grp) * a.gp + u.idx) * CP + tid] = t;
           }
-          if (tid == 0) ctl.progress = ctl.progress + 1;
+          if (tid == 0) fb_tell(ctl);
         }
       }
     }
@@ -878,7 +889,7 @@ __device__ void fb_adapt_main(const FbArgs& a, FbCtl& ctl, FbAdapt& ad, const Fb
             st_relaxed1(pp + CP, canonical(m));
           }
           __syncwarp();
-          if (tid == 0) ctl.progress = ctl.progress + 1;
+          if (tid == 0) fb_tell(ctl);
         }
         ++it;
       }

@@ -129,11 +129,15 @@ constexpr int kBarHelp = 3;     // the next step's buffers are preset
 // by warp 0.  Waits until `step` of them are, or the compute warps gave up
 // (their own waits are bounded); false then.
 __device__ __forceinline__ void tell_step(volatile int* progress, int step) {
-  if (threadIdx.x == 0) *progress = step;
+  if (threadIdx.x == 0) {
+    __threadfence_block();
+    *progress = step;
+  }
 }
 __device__ __forceinline__ bool await_step(volatile int* progress, volatile int* dead, int step) {
   bool ok = true;
   while (ok && *progress < step) ok = *dead == 0;
+  __threadfence_block();   // the compute warps' accesses before their word come first
   return __all_sync(0xffffffffu, ok);
 }
 
