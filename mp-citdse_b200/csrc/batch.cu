@@ -532,7 +532,7 @@ int horner_plan(mpc_ctx* c, int ncol) {
   const mpc_batch_state* b = c->batch;
   if (c->force_tma > 0 && b->tma_ok) return kPlanTma + std::min(c->force_tma - 1, kNumTmaShapes - 1);
   if (c->force_persist) return mpc_batch_variant(c, ncol);
-  if (c->forced_variant >= 0 && c->forced_variant < kNumVariants)
+  if (mpc_batch_pinned(c))
     return kPlanPerProduct + c->forced_variant;
   const int j = width_bucket(ncol);
   if (j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned) return b->hplan[j];
@@ -737,8 +737,12 @@ int tune(mpc_ctx* c, bool fixed, const std::vector<long long>& planned, bool all
 
 }  // namespace
 
+bool mpc_batch_pinned(const mpc_ctx* c) {
+  return c->forced_variant >= 0 && c->forced_variant < kNumVariants;
+}
+
 int mpc_batch_variant(mpc_ctx* c, int ncol) {
-  if (c->forced_variant >= 0 && c->forced_variant < kNumVariants) return c->forced_variant;
+  if (mpc_batch_pinned(c)) return c->forced_variant;
   if (c->batch) {
     const std::vector<int>& t = c->batch->tile;
     const int j = width_bucket(ncol);
@@ -875,7 +879,7 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
       std::vector<int> len(nsteps, nsteps + B);
       std::sort(len.begin(), len.end());
       for (int k = 0; k < B; ++k)   // B - k pulses run the steps (len[k-1], len[k]]
-        if (!mpc_flowb_wanted(c, B - k))
+        if (!mpc_flowb_fixed_wanted(c, B - k))
           planned[width_bucket(B - k)] += len[k] - (k ? len[k - 1] : 0);
     } else {
       double most = 0.0;
@@ -1107,7 +1111,7 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
     int act = 0;
     if ((rc = scan(&act))) break;
     if (act == 0) break;
-    if (fx.on && mpc_flowb_wanted(c, act)) {
+    if (fx.on && mpc_flowb_fixed_wanted(c, act)) {
       // the persistent batched kernels are the faster path from here on
       if (act < ncol && (rc = compact(act))) break;
       double2* in = nullptr;
@@ -1262,7 +1266,7 @@ int mpc_batch_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* 
                     "dt*max|E| = %.4g exceeds the RKF78 imaginary-axis stability bound %.4g",
                     dt * c->eps_max, kRk78ImagStability);
   CK(cudaSetDevice(c->device));
-  if (mpc_flowb_wanted(c, B))
+  if (mpc_flowb_fixed_wanted(c, B))
     return mpc_flowb_advance(c, B, pulses, t0, dt, steps, pop_index, ct, pop_out, norm_out,
                              max_steps);
   FixedStep fx{};

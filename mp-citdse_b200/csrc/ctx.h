@@ -159,6 +159,7 @@ void mpc_badj_invalidate(mpc_ctx* c);  // a setting changed: backward needs a ne
 // Stage-GEMM variant for ncol active pulses: autotuned if the context's
 // batched path has been tuned, else the default (batch.cu).
 int mpc_batch_variant(mpc_ctx* c, int ncol);
+bool mpc_batch_pinned(const mpc_ctx* c);  // MPC_BATCH_VARIANT names one
 int mpc_resident_run(mpc_ctx* c, double dt, int steps, int pop_index);
 bool mpc_use_resident(mpc_ctx* c);  // the resident path applies (set-up done, not disabled)
 bool mpc_resident_adjoint_ok(mpc_ctx* c);

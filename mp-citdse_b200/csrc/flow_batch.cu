@@ -544,12 +544,17 @@ int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb) {
   return obj_status(c, "batched adjoint pass");
 }
 
-// Whether B pulses run faster here than on the stage GEMM.
+// Whether B pulses run faster here than on the stage GEMM.  A switch that says
+// how the GEMM is to run asks for the GEMM.
 bool mpc_flowb_wanted(mpc_ctx* c, int B) {
-  if (c->path == MPC_PATH_STREAMING || !mpc_flowb_setup(c)) return false;
+  if (c->path == MPC_PATH_STREAMING || mpc_batch_pinned(c) || !mpc_flowb_setup(c)) return false;
   const mpc_flowb_state* f = c->flowb;
   const int nch = (B + CP - 1) / CP, ng = pick_groups(f, nch);
   return f->grp[ng].ok && product_us(f->grp[ng].cost, (nch + ng - 1) / ng) <= gemm_us(c->g, B);
+}
+
+bool mpc_flowb_fixed_wanted(mpc_ctx* c, int B) {
+  return !c->no_persist && !c->force_persist && !c->force_tma && mpc_flowb_wanted(c, B);
 }
 
 int mpc_flowb_states(mpc_ctx* c, int B, double2** in) {

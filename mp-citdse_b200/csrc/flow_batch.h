@@ -9,6 +9,7 @@
 
 bool mpc_flowb_setup(mpc_ctx* c);   // usable for this system
 bool mpc_flowb_wanted(mpc_ctx* c, int B);   // and the faster path for B pulses
+bool mpc_flowb_fixed_wanted(mpc_ctx* c, int B);   // idem, for fixed steps
 void mpc_flowb_free(mpc_ctx* c);
 int mpc_flowb_advance(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, double dt,
                       const int* steps, int pop_index, double* ct, double* pop_out,
