@@ -371,6 +371,8 @@ struct mpc_batch_state {
   int* cnt = nullptr;       // split-variant arrival counters (kept at zero)
   unsigned* hcnt = nullptr; // persistent Horner launch: ticket + per-column progress
   size_t hcnt_n = 0;
+  unsigned* seen = nullptr; // pinned: the status word as of event `asked`
+  cudaEvent_t asked = nullptr;
   ColState c{};
   PulseResults res{};
   std::vector<void*> allocs;
@@ -757,6 +759,8 @@ int mpc_batch_variant(mpc_ctx* c, int ncol) {
 void mpc_batch_free(mpc_ctx* c) {
   if (!c || !c->batch) return;
   for (void* p : c->batch->allocs) cudaFree(p);
+  cudaFreeHost(c->batch->seen);
+  if (c->batch->asked) cudaEventDestroy(c->batch->asked);
   delete c->batch;
   c->batch = nullptr;
 }
@@ -1107,6 +1111,32 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
     return MPC_OK;
   };
 
+  // Fixed steps: the host knows who is active, so it would queue a whole scan
+  // without looking at the status word.  Every kLookEvery steps it asks for the
+  // word, and first waits for the last answer (the steps queued since keep the
+  // GPU busy): a failure ends the call at most 2 kLookEvery steps later.
+  constexpr int kLookEvery = 64;
+  int unseen = 0;
+  bool asked = false;
+  auto look = [&](int steps) -> int {
+    unseen += steps;
+    if (unseen < kLookEvery) return MPC_OK;
+    unseen = 0;
+    if (!b->seen) CK(cudaMallocHost(&b->seen, sizeof(unsigned)));
+    if (!b->asked) CK(cudaEventCreateWithFlags(&b->asked, cudaEventDisableTiming));
+    if (asked) {
+      CK(cudaEventSynchronize(b->asked));
+      if (const unsigned st = *b->seen) {
+        CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+        return mpc_fail(MPC_ERR_DEVICE, "kernel status 0x%x in the batched propagation", st);
+      }
+    }
+    CK(cudaMemcpyAsync(b->seen, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaEventRecord(b->asked, c->stream));
+    asked = true;
+    return MPC_OK;
+  };
+
   for (;;) {
     int act = 0;
     if ((rc = scan(&act))) break;
@@ -1178,9 +1208,9 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
       }
       if (until <= 0) until = 1;
       for (long long k = 0; k + check_every <= until && rc == MPC_OK; k += check_every)
-        rc = run_group(until - k);
+        if (!(rc = run_group(until - k))) rc = look(check_every);
       for (long long k = until - until % check_every; k < until && rc == MPC_OK; ++k)
-        rc = launch_attempt();
+        if (!(rc = launch_attempt())) rc = look(1);
       if (rc || (rc = states_out())) break;
       steps_done += until;
       continue;

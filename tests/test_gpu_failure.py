@@ -157,6 +157,31 @@ def test_streamed_ring_timeout_is_reported_and_bounded(n):
         assert np.array_equal(ctx.rhs(0.3, x), want)
 
 
+@pytest.mark.parametrize("uneven", [0, 3], ids=["even", "uneven"])
+def test_batched_fixed_steps_stop_soon_after_a_failure(uneven):
+    """A pulse that is not finite from its first step on, in a scan of 4000
+    steps on the stage GEMM: the call fails after some hundred of them (the
+    status word is asked for every 64 steps, a group of 64 behind), not at the
+    end, and the next call is clean."""
+    s = random_system([40, 57, 33], gauge="l", seed=5, e_max=4.0)
+    B, p = 12, _pulse()
+    X = np.zeros((B, s.ntot), complex)
+    X[:, 0] = 1.0
+    bad = X.copy()
+    bad[3, 17] = np.nan
+    steps = [4000 - 30 * uneven * b for b in range(B)]
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.set_path("streaming")
+        Y0 = ctx.batch_advance([p] * B, 0.0, 0.1, [20] * B, X)
+        l0 = ctx.launches
+        with pytest.raises(mpc_tdse.MpcError) as ei:
+            ctx.batch_advance([p] * B, 0.0, 0.1, steps, bad)
+        assert ei.value.code == -3
+        # (tuning the width takes less than 100 steps' launches)
+        assert ctx.launches - l0 < 14 * 400
+        assert np.array_equal(ctx.batch_advance([p] * B, 0.0, 0.1, [20] * B, X), Y0)
+
+
 @pytest.mark.parametrize("path", ["streaming", "resident"])
 def test_nan_in_host_state_raises_nonfinite_status(path):
     s = random_system([40, 57, 33], gauge="v", seed=11, e_max=4.0)
