@@ -449,8 +449,10 @@ int ensure_batch(mpc_ctx* c, int B) {
       (rc = balloc(b, &s.nrm, ldc)) || (rc = balloc(b, &s.retired, ldc)) ||
       (rc = balloc(b, &s.nsteps, ldc)) ||
       (rc = balloc(b, &b->res.nacc, ldc)) || (rc = balloc(b, &b->res.nrej, ldc)) ||
-      (rc = balloc(b, &b->res.t, ldc)) || (rc = balloc(b, &b->res.status, ldc)))
+      (rc = balloc(b, &b->res.t, ldc)) || (rc = balloc(b, &b->res.status, ldc))) {
+    mpc_batch_free(c);   // the next call must not find half of the buffers
     return rc;
+  }
   // tensor maps of the TMA-fed Horner products: the coupling blocks in both
   // box shapes and the two product buffers (the library's pitches and
   // allocations satisfy TMA's 16-byte rules)

@@ -27,13 +27,17 @@ int mpc_encode_map_grouped(CUtensorMap* m, const void* base, unsigned long long 
                            unsigned long long rows, unsigned long long row_bytes,
                            unsigned box_rows, unsigned box_groups);
 
+// (an error that does not outlast its call, such as a failed allocation, is
+// cleared, or the next launch check would report it)
 #define CK(call)                                                                         \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
-    if (e_ != cudaSuccess)                                                               \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       return mpc_fail(e_ == cudaErrorMemoryAllocation ? MPC_ERR_NOMEM : MPC_ERR_CUDA,    \
                       "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__,  \
                       __LINE__);                                                         \
+    }                                                                                    \
   } while (0)
 
 struct mpc_batch_state;

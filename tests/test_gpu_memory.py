@@ -1,0 +1,65 @@
+"""Device memory: a call that does not get its work space fails with
+MPC_ERR_NOMEM and leaves the context as usable as before.  The memory is taken
+by one tensor, up to a few hundred megabytes, and given back before the check.
+"""
+import numpy as np
+import pytest
+
+import mpc_tdse
+from mpc_tdse.systems import random_system
+
+pytestmark = pytest.mark.gpu
+
+NOMEM = -4
+
+
+def _setup(B):
+    s = random_system([300] * 7, gauge="l", seed=2, e_max=8.0, d_scale=0.3)
+    Io, w = mpc_tdse.to_au(2e14, 4.0)
+    p = mpc_tdse.pulse_setup("sine", "l", Io, w, 0.0, 2, mpc_tdse.period(w, 2))
+    X = np.zeros((B, s.ntot), complex)
+    X[:, 0] = 1.0
+    return s, [p] * B, X
+
+
+def _gradient(ctx, pulses, X, B, steps):
+    return ctx.batch_objective_gradient(pulses[:B], np.full((B, 6), 1e-3), np.full(B, 2.0), 0.0,
+                                        0.1, steps, X[:B], 0, steps)
+
+
+@pytest.mark.parametrize("op,path,B", [("fixed", "streaming", 1024),
+                                       ("adaptive", "streaming", 1024),
+                                       ("gradient", "streaming", 1024), ("gradient", "auto", 32)])
+def test_context_survives_a_failed_allocation(op, path, B):
+    """1024 pulses on 2100 states: 34 MB per vector of all pulses, of which the
+    stage GEMM's work space has 18 and its gradient of 8 steps over 100; 32
+    pulses: 1 MB, and 13 of them per step of a gradient on the persistent
+    kernels."""
+    import torch
+
+    s, pulses, X = _setup(B)
+    steps = 8 if B > 32 else 80
+
+    def run(ctx, B):
+        if op == "fixed":
+            return ctx.batch_advance(pulses[:B], 0.0, 0.1, [3] * B, X[:B], history=True)
+        if op == "adaptive":
+            return ctx.batch_propagate(pulses[:B], 0.0, [0.3] * B, X[:B], dt_max=0.1)
+        return _gradient(ctx, pulses, X, B, steps)
+
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.set_path(path)
+        run(ctx, 2)   # loads the kernels
+        torch.cuda.init()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8,
+                          device="cuda")
+        with pytest.raises(mpc_tdse.MpcError) as ei:
+            run(ctx, B)
+        assert ei.value.code == NOMEM
+        del hog
+        torch.cuda.empty_cache()
+        got = run(ctx, B)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.set_path(path)
+        want = run(ctx, B)
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(got, want))
