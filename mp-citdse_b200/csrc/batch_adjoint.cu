@@ -371,10 +371,14 @@ int mpc_batch_objective(mpc_ctx* c, int B, const mpc_pulse* pulses, int K, const
   const bool flow = mpc_flowb_objective_wanted(c, B);
   if (!c->badj) c->badj = new mpc_badj_state();
   mpc_badj_state* a = c->badj;
+  // only one path's buffers are kept: either may have been sized to most of the
+  // free memory
   if (flow) {
     a->have_forward = false;
+    badj_release(a);
     if (ckpt_every <= 0 && (rc = mpc_flowb_auto_ckpt(c, B, steps, &ckpt_every))) return rc;
   } else {
+    mpc_flowb_objective_release(c);
     if ((rc = stage_setup(c->device))) return rc;
     if (ckpt_every <= 0 && (rc = auto_ckpt(c, B, steps, &ckpt_every))) return rc;
     if ((rc = ensure_badj(c, B, steps, ckpt_every))) return rc;

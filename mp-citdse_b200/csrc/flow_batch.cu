@@ -243,6 +243,26 @@ bool mpc_flowb_setup(mpc_ctx* c) {
   return f->ok;
 }
 
+void mpc_flowb_objective_release(mpc_ctx* c) {
+  mpc_flowb_state* f = c->flowb;
+  if (!f) return;
+  auto drop = [](auto** p, size_t* cap) {
+    cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+  };
+  drop(&f->oint, &f->oint_n);
+  drop(&f->oio, &f->oio_n);
+  drop(&f->oF, &f->oF_n);
+  drop(&f->onorm, &f->onorm_n);
+  drop(&f->ockp, &f->ockp_n);
+  drop(&f->oseg, &f->oseg_n);
+  drop(&f->olam, &f->olam_n);
+  drop(&f->ofs, &f->ofs_n);
+  drop(&f->ofp, &f->ofp_n);
+  drop(&f->ofb, &f->ofb_n);
+}
+
 void mpc_flowb_free(mpc_ctx* c) {
   if (!c || !c->flowb) return;
   mpc_flowb_state* f = c->flowb;
@@ -257,16 +277,7 @@ void mpc_flowb_free(mpc_ctx* c) {
   cudaFree(f->pulse);
   cudaFree(f->t0);
   cudaFree(f->hist);
-  cudaFree(f->oint);
-  cudaFree(f->oio);
-  cudaFree(f->oF);
-  cudaFree(f->onorm);
-  cudaFree(f->ockp);
-  cudaFree(f->oseg);
-  cudaFree(f->olam);
-  cudaFree(f->ofs);
-  cudaFree(f->ofp);
-  cudaFree(f->ofb);
+  mpc_flowb_objective_release(c);
   delete f;
   c->flowb = nullptr;
 }
@@ -471,6 +482,9 @@ int mpc_flowb_objective(mpc_ctx* c, int B, const double* F, double dt, int steps
   f->ong = pick_groups(f, nch);
   f->odt = dt;
   f->okept = false;
+  // a larger set does not lie beside the smaller one it replaces
+  if (f->ockp_n < vec * nseg || f->oseg_n < vec * 13 * std::min(ckpt, steps))
+    mpc_flowb_objective_release(c);
   if ((rc = grow(&f->oint, &f->oint_n, (size_t)nch * (CP + 1) + B)) ||
       (rc = grow(&f->oio, &f->oio_n, 2 * B * n)) ||
       (rc = grow(&f->oF, &f->oF_n, (size_t)steps * B)) ||

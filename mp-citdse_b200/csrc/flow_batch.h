@@ -22,6 +22,7 @@ int mpc_flowb_auto_ckpt(mpc_ctx* c, int B, int steps, int* ckpt);
 int mpc_flowb_objective(mpc_ctx* c, int B, const double* F, double dt, int steps, int ckpt,
                         const double* ct0, double2* xN);
 int mpc_flowb_objective_backward(mpc_ctx* c, int target, double* fb);
+void mpc_flowb_objective_release(mpc_ctx* c);   // its buffers (a forward pass kept is lost)
 
 int mpc_flowb_propagate(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0,
                         const double* t_end, double h0, double dt_max, double rtol, double atol,

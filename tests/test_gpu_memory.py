@@ -63,3 +63,33 @@ def test_context_survives_a_failed_allocation(op, path, B):
         ctx.set_path(path)
         want = run(ctx, B)
     assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(got, want))
+
+
+def test_batched_objective_keeps_one_path_s_buffers():
+    """The batched gradient's buffers may be sized to most of the free memory:
+    what one path held (32 pulses, 160 steps: 2.2 GB and up) is free again once
+    the other has run, and a larger set replaces a smaller one."""
+    import torch
+
+    s, pulses, X = _setup(32)
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    with mpc_tdse.Context.from_system(s) as ctx:
+        want = {}
+        for path in ("auto", "streaming"):
+            ctx.set_path(path)
+            want[path] = _gradient(ctx, pulses, X, 32, 2)
+        held = free()
+        for big, small in (("auto", "streaming"), ("streaming", "auto")):
+            ctx.set_path(big)
+            _gradient(ctx, pulses, X, 32, 160)
+            assert held - free() > 2e9
+            ctx.set_path(small)
+            got = _gradient(ctx, pulses, X, 32, 2)
+            assert abs(held - free()) < 0.2e9
+            assert all(np.array_equal(a, b) for a, b in zip(got, want[small]))
+        # the other way round in size, on one path: 160 steps replace 2
+        ctx.set_path("auto")
+        _gradient(ctx, pulses, X, 32, 2)
+        first = _gradient(ctx, pulses, X, 32, 160)
+        again = _gradient(ctx, pulses, X, 32, 160)
+        assert all(np.array_equal(a, b) for a, b in zip(first, again))
