@@ -224,7 +224,9 @@ int mpc_propagate_batch(mpc_ctx *ctx, int B, const mpc_pulse *pulses, const doub
  * depth x k split) on this context's system at widths 1, 2, 4, ... up to B pulses and
  * keeps the fastest per width for the context's later batched calls
  * (mpc_batch_propagate times a width by itself once enough steps are run at it;
- * every variant sums in the same order, so the choice never changes results).  If table is non-null it
+ * every variant sums in the same order, so the choice never changes results), and
+ * so for the ways a fixed step can run at the widths that run on the stage GEMM
+ * (mpc_batch_fixed_plan).  If table is non-null it
  * receives up to cap rows of 5 doubles: pulses, tile width (real columns),
  * pipeline depth, k split (1: the two coupled blocks of a tile run in two
  * CTAs), microseconds per right-hand side of the chosen variant.
@@ -232,16 +234,17 @@ int mpc_propagate_batch(mpc_ctx *ctx, int B, const mpc_pulse *pulses, const doub
 int mpc_batch_autotune(mpc_ctx *ctx, int B, double *table, int cap);
 
 /* How the batched fixed step (mpc_batch_advance) runs at each width on the
- * stage GEMM: once a width (1, 2, 4, ... pulses) has about 200 steps behind or
- * before it, the library times a whole step as one launch per Horner product
- * on each cp.async-fed tile variant and as one persistent launch on each
- * unsplit tile shape, and keeps the fastest (every choice gives the same
- * bits).  Rows of 5 doubles, up to cap: pulses, kind (0 one
+ * stage GEMM: by a rule on the numbers of states and pulses, unless
+ * mpc_batch_autotune has found one of the other ways faster (one launch per
+ * Horner product on each cp.async-fed tile variant, one persistent launch on each
+ * unsplit tile shape; every choice gives the same bits).  Rows of 5 doubles, up
+ * to cap, for 1, 2, 4, ... pulses: pulses, kind (0 one
  * cp.async-fed launch per product, 1 persistent, 2 one TMA-fed launch per
- * product, 3 one cp.async-fed launch per product with each tile's two
- * coupled blocks in two CTAs), tile width (real columns), ring depth,
- * microseconds per step (0 where a width has not been timed: its default).
- * Returns the number of rows (0 before any width has been timed). */
+ * product (MPC_FORCE_TMA only), 3 one cp.async-fed launch per product with each
+ * tile's two coupled blocks in two CTAs), tile width (real columns), ring depth,
+ * microseconds per step (0 where a width has not been timed).
+ * Returns the number of rows (0 before any fixed-step call on the stage GEMM or
+ * mpc_batch_autotune). */
 int mpc_batch_fixed_plan(mpc_ctx *ctx, double *table, int cap);
 
 /* Objective and gradient (new: the reference has no gradients).

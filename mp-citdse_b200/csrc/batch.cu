@@ -380,9 +380,10 @@ struct mpc_batch_state {
   // -1: not tuned)
   std::vector<int> tile;
   std::vector<double> tile_us;
-  // steps (attempts) run or planned per bucket: a bucket is tuned once there
-  // are kTuneSteps of them, since timing the variants costs about 70 steps
-  std::vector<long long> used_fixed, used_adaptive;
+  // adaptive attempts run or planned per bucket: a bucket is tuned once there
+  // are kTuneSteps of them (timing the variants costs 63 products, 5 attempts)
+  std::vector<long long> used;
+  int fixed_rows = 0;   // buckets of fixed steps run
   // fixed-step steps, per width bucket: kPlanUntuned, -1 one launch per Horner product
   // (on the right-hand-side tuner's variant), kPlanPerProduct + v one launch
   // per product on variant v, v >= 0 the persistent launch on variant v,
@@ -527,6 +528,12 @@ int launch_stage(mpc_ctx* c, const StageArgs& a) {
   return MPC_OK;
 }
 
+// The rule for a fixed step of ncol pulses.
+int default_plan(mpc_ctx* c, int ncol) {
+  const int nrt = c->batch->nrowtiles, v = default_persistent(ncol, nrt, c->g.nstate_blk);
+  return v >= 0 ? v : kPlanPerProduct + default_variant(ncol, nrt);
+}
+
 // How a fixed step of ncol pulses runs: -1 one launch per Horner product,
 // else the persistent launch (k_batch_horner) on tile variant v.  The
 // fixed-step tuner's choice when it ran, otherwise the default for the number
@@ -540,8 +547,7 @@ int horner_plan(mpc_ctx* c, int ncol) {
     return kPlanPerProduct + c->forced_variant;
   const int j = width_bucket(ncol);
   if (j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned) return b->hplan[j];
-  const int v = default_persistent(ncol, b->nrowtiles, c->g.nstate_blk);
-  return v >= 0 ? v : kPlanPerProduct + default_variant(ncol, b->nrowtiles);
+  return default_plan(c, ncol);
 }
 
 int launch_horner_persistent_v(mpc_ctx* c, int ncol, int v) {
@@ -669,8 +675,14 @@ int tune_bucket(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
 // The fixed-step tuner: times one whole step's 12 Horner products at bucket j's
 // width as one launch per product on every tile variant (the right-hand-side
 // tuner's choice need not suit the Horner epilogue) and as the persistent
-// launch on every unsplit variant, and keeps the fastest.  Every candidate
-// computes the same tiles in the same order, so the choice changes speed only.
+// launch on every unsplit variant, and takes the fastest if it beats the default
+// rule by 3 %.  Every candidate computes the same tiles in the same order, so the
+// choice changes speed only.  On request only (mpc_batch_autotune): it costs 58 to
+// 81 steps, and over a few steps it does not see what the power limit does to a
+// long run: on six systems of 1752 to 24,482 states and 6 to 256 pulses the rule
+// was within 0.5 % of its picks or ahead of them (64 pulses on 11,914: 5.44
+// against 6.19 ms per step), so that a call of 600 steps that tuned first took
+// 12 % longer for nothing.
 // (The TMA-fed launches are not among them: 720 / 428 / 189 us per step at 256 /
 // 64 / 16 pulses against 616 / 250 / 145.)  Runs on the batch's work buffers,
 // before the propagation loads its states, with unit norms in c.nrm.
@@ -680,13 +692,15 @@ int tune_bucket_fixed(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
     b->hplan.resize(j + 1, kPlanUntuned);
     b->hplan_us.resize(j + 1, 0.0);
   }
-  std::vector<int> cands = {0, 1, 2, 3, 4};
+  const int w = std::min(1 << j, b->ldc);
+  std::vector<int> cands = {default_plan(c, w), 0, 1, 2, 3, 4};
   for (int v = 0; v < kNumVariants; ++v) cands.push_back(kPlanPerProduct + v);
   const long long l0 = c->launches;
-  const int w = std::min(1 << j, b->ldc);
   double best = 1e300;
   int rc;
-  for (int v : cands) {
+  for (size_t i = 0; i < cands.size(); ++i) {
+    const int v = cands[i];
+    if (i > 0 && v == cands[0]) continue;
     double t = 0.0;
     for (int pass = 0; pass < 2; ++pass) {   // the first one warms up, and drops the slow
       const int reps = pass ? 3 : 1;
@@ -701,7 +715,7 @@ int tune_bucket_fixed(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
       if (t > 2.0 * best) break;
     }
     if (t < best) {
-      best = t;
+      best = i > 0 ? t : 0.97 * t;
       b->hplan[j] = v;
       b->hplan_us[j] = t;
     }
@@ -710,32 +724,26 @@ int tune_bucket_fixed(mpc_ctx* c, int j, cudaEvent_t e0, cudaEvent_t e1) {
   return MPC_OK;
 }
 
-// Tunes what a call is about to use: every bucket whose steps, run so far and
-// planned[j] now, reach kTuneSteps (all: whatever they are).
-int tune(mpc_ctx* c, bool fixed, const std::vector<long long>& planned, bool all) {
+// Tunes the buckets [j0, j1) for right-hand sides, or for fixed steps.
+int tune(mpc_ctx* c, bool fixed, int j0, int j1) {
   mpc_batch_state* b = c->batch;
-  std::vector<long long>& used = fixed ? b->used_fixed : b->used_adaptive;
-  if (used.size() < planned.size()) used.resize(planned.size(), 0);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  int rc = MPC_OK;
-  for (int j = 0; j < (int)planned.size() && rc == MPC_OK; ++j) {
-    used[j] += planned[j];
-    const bool have = fixed ? j < (int)b->hplan.size() && b->hplan[j] != kPlanUntuned
-                            : j < (int)b->tile.size() && b->tile[j] >= 0;
-    if (have || (!all && (planned[j] == 0 || used[j] < kTuneSteps))) continue;
-    if (!e0) {
-      CK(cudaEventCreate(&e0));
-      CK(cudaEventCreate(&e1));
-      if (fixed) {   // the first product divides by the columns' norms
-        std::vector<double> ones(b->ldc, 1.0);
-        CK(cudaMemcpyAsync(b->c.nrm, ones.data(), sizeof(double) * b->ldc, cudaMemcpyHostToDevice,
-                           c->stream));
-      }
-    }
-    rc = fixed ? tune_bucket_fixed(c, j, e0, e1) : tune_bucket(c, j, e0, e1);
+  CK(cudaEventCreate(&e0));
+  CK(cudaEventCreate(&e1));
+  if (fixed) {   // the first product divides by the columns' norms
+    std::vector<double> ones(b->ldc, 1.0);
+    CK(cudaMemcpyAsync(b->c.nrm, ones.data(), sizeof(double) * b->ldc, cudaMemcpyHostToDevice,
+                       c->stream));
   }
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
+  int rc = MPC_OK;
+  for (int j = j0; j < j1 && rc == MPC_OK; ++j) {
+    if (!fixed)
+      rc = tune_bucket(c, j, e0, e1);
+    else if (!mpc_flowb_fixed_wanted(c, std::min(1 << j, b->ldc)))   // (else not run here)
+      rc = tune_bucket_fixed(c, j, e0, e1);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
   return rc;
 }
 
@@ -809,13 +817,12 @@ int mpc_propagate_batch(mpc_ctx* c, int B, const mpc_pulse* pulses, const double
 
 int mpc_batch_fixed_plan(mpc_ctx* c, double* table, int cap) {
   if (!c || (table && cap < 0)) return mpc_fail(MPC_ERR_ARG, "bad argument");
-  if (!c->batch || c->batch->hplan.empty()) return 0;
+  if (!c->batch) return 0;
   const mpc_batch_state* b = c->batch;
-  const int rows = (int)b->hplan.size();
+  const int timed = (int)b->hplan.size(), rows = std::max(timed, b->fixed_rows);
   for (int j = 0; table && j < rows && j < cap; ++j) {
-    int v = b->hplan[j];
+    const int v = horner_plan(c, std::min(1 << j, b->ldc));
     table[5 * j + 0] = std::min(1 << j, b->ldc);
-    if (v == kPlanUntuned) v = horner_plan(c, std::min(1 << j, b->ldc));
     if (v >= kPlanPerProduct) {
       const TileVariant& tv = kVariants[v - kPlanPerProduct];
       table[5 * j + 1] = tv.split ? 3 : 0;
@@ -831,7 +838,7 @@ int mpc_batch_fixed_plan(mpc_ctx* c, double* table, int cap) {
       table[5 * j + 2] = kVariants[vv].bn;
       table[5 * j + 3] = v >= 0 ? (kVariants[vv].nst >= 6 ? 3 : 2) : kVariants[vv].nst;
     }
-    table[5 * j + 4] = b->hplan_us[j];
+    table[5 * j + 4] = j < timed ? b->hplan_us[j] : 0.0;
   }
   return rows;
 }
@@ -841,7 +848,11 @@ int mpc_batch_autotune(mpc_ctx* c, int B, double* table, int cap) {
   CK(cudaSetDevice(c->device));
   int rc;
   if ((rc = ensure_batch(c, B))) return rc;
-  if ((rc = tune(c, false, std::vector<long long>(width_bucket(B) + 1, 0), true))) return rc;
+  const int top = width_bucket(B) + 1;
+  if ((rc = tune(c, false, 0, top))) return rc;
+  if (!c->no_persist && !c->force_persist && !c->force_tma && !mpc_batch_pinned(c) &&
+      (rc = tune(c, true, 0, top)))
+    return rc;
   const mpc_batch_state* b = c->batch;
   const int rows = (int)b->tile.size();
   for (int j = 0; table && j < rows && j < cap; ++j) {
@@ -875,24 +886,20 @@ int batch_run(mpc_ctx* c, int B, const mpc_pulse* pulses, const double* t0, cons
 
   if (fx.on && c->force_tma > 0 && !b->tma_ok)
     return mpc_fail(MPC_ERR_CUDA, "MPC_FORCE_TMA: the TMA tensor maps could not be set up");
-  // the tuners run on the work buffers, before the states are loaded; what each
-  // width is about to run is known for fixed steps, and bounded from below by
-  // the longest pulse's steps of dt_max for adaptive ones
-  if (!std::getenv("MPC_NO_AUTOTUNE") &&
-      !(fx.on && (c->no_persist || c->force_persist || c->force_tma))) {
-    std::vector<long long> planned(width_bucket(B) + 1, 0);
-    if (fx.on) {
-      std::vector<int> len(nsteps, nsteps + B);
-      std::sort(len.begin(), len.end());
-      for (int k = 0; k < B; ++k)   // B - k pulses run the steps (len[k-1], len[k]]
-        if (!mpc_flowb_fixed_wanted(c, B - k))
-          planned[width_bucket(B - k)] += len[k] - (k ? len[k - 1] : 0);
-    } else {
-      double most = 0.0;
-      for (int k = 0; k < B; ++k) most = std::max(most, t_end[k] - t0[k]);
-      planned.back() = (long long)std::min(most / dt_max, 1e6);
-    }
-    if ((rc = tune(c, fx.on, planned, false))) return rc;
+  // adaptive steps: the tuner runs on the work buffers, before the states are
+  // loaded; the attempts are bounded from below by the longest pulse's steps of
+  // dt_max
+  const int bucket = width_bucket(B);
+  if (fx.on) {
+    b->fixed_rows = std::max(b->fixed_rows, bucket + 1);
+  } else if (!std::getenv("MPC_NO_AUTOTUNE")) {
+    double most = 0.0;
+    for (int k = 0; k < B; ++k) most = std::max(most, t_end[k] - t0[k]);
+    if ((int)b->used.size() <= bucket) b->used.resize(bucket + 1, 0);
+    b->used[bucket] += (long long)std::min(most / dt_max, 1e6);
+    const bool have = bucket < (int)b->tile.size() && b->tile[bucket] >= 0;
+    if (!have && b->used[bucket] >= kTuneSteps && (rc = tune(c, false, bucket, bucket + 1)))
+      return rc;
   }
 
   // per-column start state

@@ -289,7 +289,8 @@ class Context:
         return out.view(np.complex128).reshape(B, -1)
 
     def batch_autotune(self, B):
-        """Tunes the batched GEMM tiles up to B pulses; returns rows of
+        """Tunes the batched GEMM, right-hand sides and fixed steps, up to B
+        pulses; returns rows, for the right-hand sides, of
         (pulses, tile width in real columns, pipeline depth, k split, us per RHS)."""
         cap = 32
         tab = np.zeros((cap, 5))
@@ -299,9 +300,10 @@ class Context:
 
     def batch_fixed_plan(self):
         """Rows of (pulses, kind, tile width, ring depth, us per step) chosen
-        for the batched fixed step; kind 0: one cp.async-fed launch per
-        Horner product, 1: one persistent launch, 2: one TMA-fed launch per
-        product, 3: as 0 with each tile's coupled blocks in two CTAs."""
+        for the batched fixed step on the stage GEMM (us 0 where not timed, see
+        batch_autotune); kind 0: one cp.async-fed launch per Horner product, 1:
+        one persistent launch, 2: one TMA-fed launch per product, 3: as 0 with
+        each tile's coupled blocks in two CTAs."""
         cap = 32
         tab = np.zeros((cap, 5))
         r = lib().mpc_batch_fixed_plan(self._h, _ptr(tab), cap)
