@@ -854,8 +854,8 @@ int mpc_batch_autotune(mpc_ctx* c, int B, double* table, int cap) {
       (rc = tune(c, true, 0, top)))
     return rc;
   const mpc_batch_state* b = c->batch;
-  const int rows = (int)b->tile.size();
-  for (int j = 0; table && j < rows && j < cap; ++j) {
+  // (wider buckets may be there too, those between perhaps not tuned)
+  for (int j = 0; table && j < top && j < cap; ++j) {
     const int v = b->tile[j];
     table[5 * j + 0] = std::min(1 << j, b->ldc);
     table[5 * j + 1] = kVariants[v].bn;
@@ -863,7 +863,7 @@ int mpc_batch_autotune(mpc_ctx* c, int B, double* table, int cap) {
     table[5 * j + 3] = kVariants[v].split;
     table[5 * j + 4] = b->tile_us[(size_t)j * kNumVariants + v];
   }
-  return rows;
+  return top;
 }
 
 }  // extern "C"
