@@ -454,10 +454,10 @@ int ensure_batch(mpc_ctx* c, int B) {
     mpc_batch_free(c);   // the next call must not find half of the buffers
     return rc;
   }
-  // tensor maps of the TMA-fed Horner products: the coupling blocks in both
-  // box shapes and the two product buffers (the library's pitches and
-  // allocations satisfy TMA's 16-byte rules)
-  {
+  // tensor maps of the TMA-fed Horner products, which only MPC_FORCE_TMA asks
+  // for: the coupling blocks in both box shapes and the two product buffers (the
+  // library's pitches and allocations satisfy TMA's 16-byte rules)
+  if (c->force_tma > 0) {
     static bool attrs_set[64] = {};
     if (c->device >= 0 && c->device < 64 && !attrs_set[c->device]) {
       CK(set_tma_attrs());
