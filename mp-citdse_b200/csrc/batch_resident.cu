@@ -4,11 +4,13 @@
 //
 // When a batch has narrowed to at most 8 pulses, the streamed GEMM path
 // (batch.cu) is bound by per-launch latency rather than by work.  This kernel
-// takes over instead, for the systems that the persistent batched kernels
-// (flow_batch.cu) have no layout for and that fit shared memory all the same.  Each of G CTAs (one per SM) owns a contiguous range of
-// rows of one state block L and keeps their coupling rows in shared memory
-// for the whole run (column r of D_{L-1} and row r of D_L, the latter
-// negated in the velocity gauge), as the single-pulse resident kernel does.
+// takes over instead where the persistent batched kernels (flow_batch.cu) have
+// not: on systems they have no layout for (a window of more than 800 states)
+// that fit shared memory all the same, in an adaptive batch that began too wide
+// for them, and where a switch keeps a batch on the GEMM.  Each of G CTAs (one
+// per SM) owns a contiguous range of rows of one state block L and keeps their
+// coupling rows in shared memory for the whole run (column r of D_{L-1} and row
+// r of D_L, the latter negated in the velocity gauge).
 // Per stage a CTA loads the stage input of the two blocks its rows couple to
 // for all P pulse columns (L2), forms the coupling sums for all its rows at
 // once (each window element is read once from shared memory and applied to
