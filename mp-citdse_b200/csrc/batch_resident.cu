@@ -643,9 +643,7 @@ int mpc_batch_res_pmax(mpc_ctx* c) {
     }
     if (need + static_bytes > (size_t)optin) break;
     const void* k = br_kernel_for(P);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) !=
-        cudaSuccess)
-      break;
+    if (!mpc_allow_smem(k, optin)) break;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, QT, need) != cudaSuccess ||
         per_sm < 1)

@@ -133,6 +133,17 @@ def test_resident_kernel_adaptive_steps(n, B):
         assert np.array_equal(Y[1], X[1])
 
 
+def test_resident_kernel_in_two_contexts_of_different_size():
+    """The kernel's shared-memory limit belongs to the function: a second,
+    smaller system must not take it from the first."""
+    big, pb, Xb = _case(NO_LAYOUT, "l", 2)
+    small, ps, Xs = _case([401, 30, 402], "l", 2)
+    with mpc_tdse.Context.from_system(big) as a, mpc_tdse.Context.from_system(small) as b:
+        Y0 = a.batch_advance(pb, 0.0, 0.1, [4, 5], Xb)
+        b.batch_advance(ps, 0.0, 0.1, [4, 5], Xs)
+        assert np.array_equal(a.batch_advance(pb, 0.0, 0.1, [4, 5], Xb), Y0)
+
+
 # ---- failures ----
 
 @pytest.mark.parametrize("op,n,B", [("fixed", [60, 70, 50], 9), ("fixed", [97] * 5, 20),
