@@ -146,6 +146,7 @@ struct mpc_badj_state {
   double dt = 0.0;
   std::vector<double> T, u, tn;
   bool have_forward = false;
+  bool last_kept = false;    // segX / segY hold the last segment
   bool flow = false;         // the last forward ran on the persistent kernels (flow_batch.cu)
   // device buffers ([n][ldc] complex unless noted)
   double2* ckpts = nullptr;  // [nseg + 1]
@@ -488,6 +489,7 @@ int mpc_batch_objective(mpc_ctx* c, int B, const mpc_pulse* pulses, int K, const
     J[b] = y;
   }
   a->have_forward = true;
+  a->last_kept = true;
   return MPC_OK;
 }
 
@@ -524,12 +526,14 @@ int mpc_batch_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
     CK(cudaGetLastError());
     ++c->launches;
     const double hb12 = a->dt * rkf78::B8[kNumStages - 1];
+    const bool kept = a->last_kept;
+    a->last_kept = kept && a->nseg == 1;   // recomputing a segment overwrites it
     for (int seg = a->nseg - 1; seg >= 0; --seg) {
       const int n0 = seg * ckpt;
       const int len = std::min(ckpt, steps - n0);
-      // recompute the segment (the last one is still resident from the
+      // recompute the segment (the last one may still be there from the
       // forward pass): states, stage inputs and norms
-      if (seg < a->nseg - 1) {
+      if (!kept || seg < a->nseg - 1) {
         CK(cudaMemcpyAsync(a->segX, a->ckpts + slab * seg, sizeof(double2) * slab,
                            cudaMemcpyDeviceToDevice, c->stream));
         for (int j = 0; j < len; ++j)

@@ -100,7 +100,7 @@ def test_2e_yield_and_central_difference():
 
 def test_checkpoint_interval_and_reallocation_are_bit_identical():
     """Intervals that make the work buffers grow and shrink between calls, on 35
-    columns; 0: sized to the free memory."""
+    columns; 0: sized to the free memory; a second reverse pass."""
     s = random_system([100, 130, 65], gauge="v", seed=3, e_max=8.0, d_scale=0.3)
     pulses, U, T = _batch("v", 35, K=24, seed=9)
     X0 = np.zeros((35, s.ntot), complex)
@@ -110,5 +110,7 @@ def test_checkpoint_interval_and_reallocation_are_bit_identical():
         r = []
         for c in (64, 9, 500, 100, 1, 0):
             r.append(ctx.batch_objective_gradient(pulses, U, T, 0.0, 0.1, 101, X0, 0, ckpt_every=c))
+            G2, Fb2 = ctx.batch_objective_backward()
+            assert np.array_equal(G2, r[-1][1]) and np.array_equal(Fb2, r[-1][2])
     for got in r[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(got, r[0]))
