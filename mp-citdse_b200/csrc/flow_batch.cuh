@@ -562,7 +562,8 @@ __device__ void fb_fixed_helper(const FbArgs& a, FbCtl& ctl, const FbView& u, in
           ctl.t[c][q] += a.dt;
           if (u.idx == 0) {
             if (a.norm_hist) a.norm_hist[(long long)id * a.hist_ld + n] = nrm;
-            if (!(nrm > 0.0) || !isfinite(nrm)) atomicOr(a.status, ST_NONFINITE);
+            // (the objective gives such a pulse its NaN, beside the others' numbers)
+            if (!a.seg_v && (!(nrm > 0.0) || !isfinite(nrm))) atomicOr(a.status, ST_NONFINITE);
           }
         }
         ctl.nrm[c][q] = make_double2(nrm, 1.0 / nrm);

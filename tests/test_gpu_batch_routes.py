@@ -178,3 +178,47 @@ def test_wait_that_runs_out_is_reported(op, n, B):
         assert ei.value.code == -3
         ctx.set_wait_limit(2.0)
         assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(run(ctx), want))
+
+
+@pytest.mark.parametrize("path", ["auto", "streaming"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_pulse_beside_finite_ones(bad, path):
+    """Fixed steps fail as a whole; an adaptive pulse that is not finite gives up
+    alone: the call reports it, and the others' states, counts and times are
+    written; the objective and its gradient are NaN for that pulse.  The others
+    have the bits they have beside a finite pulse."""
+    import ctypes as C
+
+    s, pulses, X = _case([97] * 5, "l", 12)
+    Xbad = X.copy()
+    Xbad[4, 200] = bad
+    U, T = np.full((12, 6), 1e-3), np.full(12, 2.0)
+    dp, ip = C.POINTER(C.c_double), C.POINTER(C.c_int)
+    arr = (mpc_tdse.Pulse * 12)(*pulses)
+    t0, te = np.zeros(12), 0.3 + 0.05 * np.arange(12)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.set_path(path)
+
+        def adaptive(x):
+            xf = x.view(np.float64).copy()
+            acc, rej, tf = np.zeros(12, np.int32), np.zeros(12, np.int32), np.zeros(12)
+            rc = mpc_tdse.lib().mpc_batch_propagate(
+                ctx._h, 12, arr, t0.ctypes.data_as(dp), te.ctypes.data_as(dp), 0.05, 0.2, 1e-10,
+                1e-10, 0, xf.ctypes.data_as(dp), acc.ctypes.data_as(ip), rej.ctypes.data_as(ip),
+                tf.ctypes.data_as(dp))
+            return rc, xf.view(np.complex128), acc, rej, tf
+
+        with pytest.raises(mpc_tdse.MpcError) as ei:
+            ctx.batch_advance(pulses, 0.0, 0.1, [5] * 12, Xbad)
+        assert ei.value.code == -3
+        rc, Y, acc, rej, tf = adaptive(Xbad)
+        rc0, Y0, acc0, rej0, tf0 = adaptive(X)
+        assert rc == -3 and rc0 == 0
+        ok = np.arange(12) != 4
+        grads = [ctx.batch_objective_gradient(pulses, U, T, 0.0, 0.1, 5, x, 0, 2) for x in (Xbad, X)]
+        for a, b in zip(*grads):
+            assert np.array_equal(a[ok], b[ok]) and np.all(np.isfinite(b))
+            assert np.all(np.isnan(a[4]) | (a[4] == 0.0)) and np.any(np.isnan(a[4]))
+        for a, b in ((Y, Y0), (acc, acc0), (rej, rej0), (tf, tf0)):
+            assert np.array_equal(a[ok], b[ok])
+        assert acc[4] == 0 and tf[4] == 0.0
