@@ -228,7 +228,9 @@ struct FbTile {
 #pragma unroll
         for (int i = 0; i < BD; ++i)
           if (nb * BD + i < KT && nb * BD + i < nj) miss = miss || missing(y[i]);
-        if (!__any_sync(0xffffffffu, miss) || *dead) break;
+        if (!__any_sync(0xffffffffu, miss)) break;
+        // (by vote: the word may change between two lanes' reads)
+        if (__any_sync(0xffffffffu, *dead != 0)) break;
 #pragma unroll
         for (int i = 0; i < BD; ++i)
           if (nb * BD + i < KT && nb * BD + i < nj && missing(y[i]))
