@@ -282,9 +282,10 @@ struct mpc_adjoint_state {
   double2* segX = nullptr;    // [ckpt + 1][ntot]
   double2* segY = nullptr;    // [ckpt][13][ntot]  (slot 0 unused: y_0 = x_n)
   double* segN = nullptr;     // [ckpt]
-  // resident passes: a second segment buffer set (recompute of one segment
-  // while the one after it is swept) and every step's norm, allocated on
-  // first use; a segment's slots hold its Horner vectors and states
+  // resident passes: every step's norm, and for a reverse pass of more than one
+  // segment a second buffer set (recompute of one segment while the one after it
+  // is swept; the last segment is in segY), allocated on first use; a segment's
+  // slots hold its Horner vectors and states
   double2* segY2 = nullptr;
   double* norms = nullptr;
   double2* lam = nullptr;
@@ -352,13 +353,6 @@ int ensure_adjoint(mpc_ctx* c, int steps, int ckpt) {
   a->cap_seg = ckpt;
   a->cap_steps = steps;
   return MPC_OK;
-}
-
-int ensure_resident(mpc_adjoint_state* a, size_t n) {
-  int rc = MPC_OK;
-  if (!a->segY2) rc = aalloc(a, &a->segY2, n * a->cap_seg * kNumStages);
-  if (!rc && !a->norms) rc = aalloc(a, &a->norms, a->cap_steps);
-  return rc;
 }
 
 // One forward step from x (stage inputs into ys[1..12], x_new into ys[13]),
@@ -435,10 +429,9 @@ int mpc_objective(mpc_ctx* c, const mpc_pulse* p, int K, const double* u, double
   if (a->resident) {
     // one persistent launch; it stores the checkpoints as it passes them, and
     // the last segment's vectors, which the reverse pass then need not recompute
-    if ((rc = ensure_resident(a, n)) ||
-        (rc = mpc_resident_forward_ex(c, a->ckpts, a->ckpts + n * a->nseg, c->d_Ftab, dt, steps,
-                                      a->norms, a->ckpts, ckpt_every,
-                                      ((a->nseg - 1) & 1) ? a->segY2 : a->segY,
+    if (!a->norms && (rc = aalloc(a, &a->norms, a->cap_steps))) return rc;
+    if ((rc = mpc_resident_forward_ex(c, a->ckpts, a->ckpts + n * a->nseg, c->d_Ftab, dt, steps,
+                                      a->norms, a->ckpts, ckpt_every, a->segY,
                                       (a->nseg - 1) * ckpt_every, (long long)n)))
       return rc;
   } else {
@@ -535,7 +528,11 @@ int mpc_objective_backward(mpc_ctx* c, double* grad_u, double* dJdF) {
   if (a->resident) {
     // one persistent launch: each segment's recompute runs concurrently with
     // the sweep of the segment after it
-    double2* sv[2] = {a->segY, a->segY2};
+    if (nseg > 1 && !a->segY2 && (rc = aalloc(a, &a->segY2, n * a->cap_seg * kNumStages)))
+      return rc;
+    double2* sv[2];
+    sv[(nseg - 1) & 1] = a->segY;
+    sv[nseg & 1] = a->segY2;
     if ((rc = mpc_resident_backward(c, a->ckpts, a->norms, steps, ckpt, c->d_Ftab, dt, sv,
                                     a->last_kept, a->lam, a->fbar, (long long)n)))
       return rc;

@@ -93,3 +93,27 @@ def test_batched_objective_keeps_one_path_s_buffers():
         first = _gradient(ctx, pulses, X, 32, 160)
         again = _gradient(ctx, pulses, X, 32, 160)
         assert all(np.array_equal(a, b) for a, b in zip(first, again))
+
+
+def test_objective_without_gradient_holds_one_segment():
+    """Two segments of 10,000 steps on 180 states (0.41 GB each): the objective
+    alone takes the memory of one, and the gradient has the bits of another
+    interval's."""
+    import torch
+
+    s = random_system([60, 70, 50], gauge="l", seed=2, e_max=8.0, d_scale=0.3)
+    Io, w = mpc_tdse.to_au(2e14, 4.0)
+    p = mpc_tdse.pulse_setup("sine", "l", Io, w, 0.0, 2, mpc_tdse.period(w, 2))
+    x = np.zeros(s.ntot, complex)
+    x[0] = 1.0
+    u = np.full(6, 1e-3)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        want = ctx.objective_gradient(p, u, 2.0, 0.0, 0.1, 20000, x, 0, 64)
+        ctx.objective(p, u, 2.0, 0.0, 0.1, 3, x, 0, 2)
+    with mpc_tdse.Context.from_system(s) as ctx:
+        ctx.objective_gradient(p, u, 2.0, 0.0, 0.1, 3, x, 0, 2)   # loads the kernels
+        free = torch.cuda.mem_get_info()[0]
+        J = ctx.objective(p, u, 2.0, 0.0, 0.1, 20000, x, 0, 10000)
+        assert free - torch.cuda.mem_get_info()[0] < 0.6e9
+        g = ctx.objective_backward()
+    assert J == want[0] and all(np.array_equal(a, b) for a, b in zip(g, want[1:]))
