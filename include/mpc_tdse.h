@@ -109,9 +109,8 @@ int mpc_ctx_set_wait_limit(mpc_ctx *ctx, double seconds);
 /* Fault injection for tests of the failure detection above: the next
  * persistent launch on this context gets arrival targets one beyond what its
  * CTAs can make, or, if it comes first, the next launch of the streaming kernel
- * waits for 16 bytes more than its first loads bring: the first such wait runs
- * out after its limit and the call reports the timeout.  Later launches are
- * normal. */
+ * a first tile that waits for one: the first such wait runs out after its limit
+ * and the call reports the timeout.  Later launches are normal. */
 int mpc_ctx_inject_barrier_timeout(mpc_ctx *ctx);
 
 /* Total number of states sum(state_sz). */

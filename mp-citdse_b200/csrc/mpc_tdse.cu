@@ -260,7 +260,7 @@ namespace {
 
 int mpc_launch_stream(mpc_ctx* c, const double2* y) {
   c->sargs.y = y;
-  c->sargs.tx_skew = 16u * (unsigned)mpc_barrier_cfg(c).skew;
+  c->sargs.skew = (unsigned)mpc_barrier_cfg(c).skew;
   ProfScope ps(c, MPC_KERNEL_RHS_STREAM);
   CK(mpc_launch_pdl(k_rhs_stream, dim3(c->stream_grid), dim3(kStreamThreads), kStreamSmem,
                     c->stream, c->sargs, c->tmaps));

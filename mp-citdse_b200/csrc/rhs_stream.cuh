@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 1 + (s == 0 ? a.skew : 0u));
       mbar_init(&empty[s], kConsumerWarps);
     }
     fence_mbar_init();
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     for (int i = 0; i < pre; ++i) {
       int b, s, rt;
       decode_tile(g, t_begin + i, b, s, rt);
-      mbar_arrive_expect_tx(&full[i], kTileBytes + kYRowBytes + (i == 0 ? a.tx_skew : 0u));
+      mbar_arrive_expect_tx(&full[i], kTileBytes + kYRowBytes);
       tma_load_2d_hint(tiles + i * (kTileR * kStripW), &tm.m[b], &full[i], s * kStripW,
                        rt * kTileR, t_begin + i < keep_end ? keep_policy : stream_policy);
     }

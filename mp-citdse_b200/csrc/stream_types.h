@@ -21,9 +21,9 @@ struct StreamArgs {
   // the first keep_frac of every CTA's tiles are loaded with an L2 evict-last
   // hint (they stay in L2 from pass to pass), the rest evict-first
   float keep_frac;
-  // 0; else bytes more than its load brings that each CTA's first tile waits for
-  // (a test's wait that runs out)
-  unsigned tx_skew;
+  // 0; 1 in a test of a wait that runs out: each CTA's first tile waits for one
+  // more arrival than there is
+  unsigned skew;
   Geometry g;
 };
 

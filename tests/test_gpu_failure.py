@@ -177,7 +177,7 @@ def test_batched_fixed_steps_stop_soon_after_a_failure(uneven):
         with pytest.raises(mpc_tdse.MpcError) as ei:
             ctx.batch_advance([p] * B, 0.0, 0.1, steps, bad)
         assert ei.value.code == -3
-        # (tuning the width takes less than 100 steps' launches)
+        # (a step takes 13 launches, or 14)
         assert ctx.launches - l0 < 14 * 400
         assert np.array_equal(ctx.batch_advance([p] * B, 0.0, 0.1, [20] * B, X), Y0)
 
