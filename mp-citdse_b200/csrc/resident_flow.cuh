@@ -33,11 +33,11 @@
 // window, and the window's elements are divided as they enter the next step
 // (by every reader alike, so a run cut into several calls has the same bits).
 //
-// Measured, per step: 1752 states (6 blocks of 292) 22.0 us, 3480 states (9
-// blocks of 384-388) 30.5 us, against 64.9 and 89.5 us for 13 stages with a grid
+// Measured, per step: 1752 states (6 blocks of 292) 20.9 us (22.0 before the
+// fences at the spins), 3480 states (9 blocks of 384-388) 30.4 us, against 64.9 and 89.5 us for 13 stages with a grid
 // barrier each and every row re-reading the window from shared memory; a
 // gradient of 192 steps (3492 states) 14.4 ms against 45.6 ms.  Of a product's
-// 3,560 cycles at 1752 states about 2,600 are the exchange (publish, poll, the
+// 3,560 cycles at 1752 states and 22.0 us about 2,600 are the exchange (publish, poll, the
 // slowest of a CTA's polls), 690 the sums, 500 the row update.  Tried: two FMA
 // chains per sum (no change), a pause of 50 ns between polls (+5 %), a delay
 // of 400 / 800 / 1200 cycles before the first poll (-3 / +2 / +12 %).
